@@ -14,9 +14,8 @@
 #include "kernels.cuh"
 #include "pcg64.cuh"
 
-void exm_make_tmap(exm_ctx *ctx);
 void exm_store_generate(exm_ctx *ctx, int k, const float *M, const float *P, const float *Q, float S, uint32_t seed);
-void exm_run_node_values(exm_ctx *ctx, exm_slot &sl, double *d_lamN);
+void exm_run_node_values(exm_ctx *ctx, exm_slot &sl, int m_base, int nmc, double *d_lamN);
 void exm_run_distance_weights_y(exm_ctx *ctx, const double *d_y, double ymin, int prior, const double *d_lny,
                                 const double *d_p, int n_dens, const double *d_gl);
 void exm_run_topk(exm_ctx *ctx, exm_slot &sl, int nmc, const int *d_order_chunk, int K, int S);
@@ -65,8 +64,8 @@ void exm_ensure(exm_ctx *ctx, dbuf &b, size_t bytes)
 
 static void free_slot(exm_ctx *ctx, exm_slot &s)
 {
-    dbuf *all[] = {&s.traj, &s.trajlo, &s.fft, &s.keys, &s.picks, &s.rej, &s.sel, &s.hist, &s.win, &s.cnt,
-                   &s.desc, &s.tside, &s.part, &s.lnl, &s.lnb, &s.dev_err, &s.din};
+    dbuf *all[] = {&s.traj, &s.trajlo, &s.keys, &s.picks, &s.rej, &s.sel, &s.hist, &s.win, &s.cnt,
+                   &s.desc, &s.tside, &s.part, &s.lamN, &s.lnl, &s.lnb, &s.dev_err, &s.din};
     for (dbuf *b : all) exm_free(ctx, *b);
     if (s.hostin.p) cudaFreeHost(s.hostin.p);
     s.hostin.p = nullptr;
@@ -298,8 +297,6 @@ extern "C" int exm_ctx_create_sharing(exm_ctx *parent, size_t hbm_budget, exm_ct
         ctx->d_tscale.p = parent->d_tscale.p;
         ctx->tstride = parent->tstride;
         ctx->d_tau.p = parent->d_tau.p;
-        ctx->tmap = parent->tmap;
-        ctx->tmap_ok = parent->tmap_ok;
         ctx->gather_cfg = parent->gather_cfg;
         ctx->gather_chunk_pct = parent->gather_chunk_pct;
         ctx->traj_fp64 = parent->traj_fp64;
@@ -515,7 +512,6 @@ extern "C" int exm_store_init(exm_ctx *ctx, int n_nodes, int ntau, int nphif, in
     for (int r = 0; r < ntau; ++r) t32[r] = (int)tau_idx[r];
     exm_ensure(ctx, ctx->d_tau, sizeof(int) * ntau);
     EXM_CUDA(cudaMemcpy(ctx->d_tau.p, t32.data(), sizeof(int) * ntau, cudaMemcpyHostToDevice));
-    exm_make_tmap(ctx);
     exm_ensure(ctx, ctx->d_stats, 4 * sizeof(unsigned long long));
     EXM_CUDA(cudaMemsetAsync(ctx->d_stats.p, 0, 4 * sizeof(unsigned long long), ctx->stream));
     EXM_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -869,9 +865,37 @@ extern "C" int exm_pe_prepare(exm_ctx *ctx, double ymin, int prior, const double
 // ------------------------------------------------------------------ the per-segment pipeline
 
 struct RunShape {
-    int K, S, nwalk, use_sel, nmc_max, rc;
+    int K, S, nwalk, use_sel, nmc_max, rc, nparts;
     float lw;
 };
+
+// lags per pass (descriptors and time indices of at most 8 GiB) and parts of the plane pairs per block
+static void plan_lags(exm_ctx *ctx, RunShape &rs)
+{
+    const size_t per_lag = (size_t)rs.nmc_max * rs.nwalk * 20;
+    const size_t cap = (size_t)8 << 30;
+    rs.rc = (int)std::max<size_t>(1, std::min<size_t>((size_t)ctx->ntau, cap / std::max<size_t>(per_lag, 1)));
+    rs.nparts = exm_gather_parts(ctx, rs.nmc_max, 0, rs.nwalk, rs.rc);
+}
+
+// the buffers of the tap build and the gather
+static void ensure_taps(exm_ctx *ctx, exm_slot &sl, const RunShape &rs)
+{
+    const size_t pitch = (size_t)exm_desc_pitch(rs.nmc_max, rs.nwalk);
+    // offsets, and the counts of the parts of the walked times (the parts of a smaller last pass: 32 at most)
+    size_t parts = 0;
+    for (int nmc : {rs.nmc_max, ctx->nm % rs.nmc_max})
+        for (int rc : {rs.rc, ctx->ntau % rs.rc}) {
+            if (nmc <= 0 || rc <= 0) continue;
+            const int nq = exm_tap_parts(ctx, nmc, rs.nwalk, rc);
+            if (nq > 1) parts = std::max(parts, (size_t)nq * rc * nmc);
+        }
+    exm_ensure(ctx, sl.cnt, EXM_NPAIR * ((size_t)rs.rc * (rs.nmc_max + 1) + parts) * sizeof(int));
+    exm_ensure(ctx, sl.desc, (size_t)rs.rc * pitch * sizeof(uint4));
+    exm_ensure(ctx, sl.tside, (size_t)rs.rc * pitch * sizeof(int32_t));
+    exm_ensure(ctx, sl.part, (size_t)(ctx->nn + 1) * ctx->ntau * rs.nparts * ctx->nm * sizeof(double));
+    sl.nparts = rs.nparts;
+}
 
 static RunShape run_shape(exm_ctx *ctx, int K, int S)
 {
@@ -894,9 +918,7 @@ static RunShape run_shape(exm_ctx *ctx, int K, int S)
         rs.lw = 0.f;
     }
     rs.nmc_max = std::min(ctx->nm, EXM_MAX_CHUNK);
-    const size_t per_lag = (size_t)rs.nmc_max * rs.nwalk * 20;
-    const size_t cap = (size_t)8 << 30;
-    rs.rc = (int)std::max<size_t>(1, std::min<size_t>((size_t)ctx->ntau, cap / std::max<size_t>(per_lag, 1)));
+    plan_lags(ctx, rs);
     return rs;
 }
 
@@ -905,7 +927,7 @@ static void ensure_slot(exm_ctx *ctx, exm_slot &sl, const RunShape &rs)
     const size_t nmc = rs.nmc_max, nt = ctx->nt, nf = ctx->nfreq;
     exm_ensure(ctx, sl.traj, 2 * nmc * nt * sizeof(float2));
     if (ctx->traj_fp64) exm_ensure(ctx, sl.trajlo, 2 * nmc * nt * sizeof(float));
-    exm_ensure(ctx, sl.fft, 2 * nmc * nt * sizeof(double2));
+    exm_ensure(ctx, sl.desc, 2 * nmc * nt * sizeof(double2));   // the filter's buffer before it holds descriptors
     const size_t n_draws = rs.K > 0 ? (((size_t)ctx->nm * rs.S + EXM_MAX_REJ + 63) / 64) * 64 : 0;
     exm_ensure(ctx, sl.keys, std::max<size_t>(rs.K > 0 ? nmc * nt : 1, n_draws) * sizeof(uint32_t));
     exm_ensure(ctx, sl.picks, std::max<size_t>(1, (size_t)ctx->nm * rs.S) * sizeof(int32_t));
@@ -913,11 +935,8 @@ static void ensure_slot(exm_ctx *ctx, exm_slot &sl, const RunShape &rs)
     exm_ensure(ctx, sl.sel, std::max<size_t>(1, rs.use_sel ? nmc * rs.nwalk : 1) * sizeof(int32_t));
     exm_ensure(ctx, sl.hist, (EXM_HB_N + 256) * sizeof(int));
     exm_ensure(ctx, sl.win, (2 + EXM_MAX_NODES) * sizeof(int));
-    exm_ensure(ctx, sl.cnt, (size_t)rs.rc * EXM_NPAIR * (nmc + 1) * sizeof(int));
-    const size_t pitch = (size_t)exm_desc_pitch((long long)nmc * rs.nwalk);
-    exm_ensure(ctx, sl.desc, (size_t)rs.rc * pitch * sizeof(uint4));
-    exm_ensure(ctx, sl.tside, (size_t)rs.rc * pitch * sizeof(int32_t));
-    exm_ensure(ctx, sl.part, (size_t)(ctx->nn + 1) * ctx->ntau * ctx->nm * sizeof(double));
+    ensure_taps(ctx, sl, rs);
+    exm_ensure(ctx, sl.lamN, (size_t)(ctx->nn + 1) * ctx->nm * sizeof(double));
     exm_ensure(ctx, sl.lnl, (size_t)ctx->nm * sizeof(double));
     exm_ensure(ctx, sl.lnb, sizeof(double));
     exm_ensure(ctx, sl.dev_err, sizeof(unsigned));
@@ -1448,14 +1467,9 @@ extern "C" int exm_node_values(exm_ctx *ctx, double *lamN_out)
     rs.nwalk = ctx->times_ok ? ctx->cur_nwalk : ctx->nt;
     rs.use_sel = ctx->times_ok ? 1 : 0;
     rs.lw = ctx->cur_lw;
-    const size_t per_lag = (size_t)ctx->nm * rs.nwalk * 20;
-    rs.rc = (int)std::max<size_t>(1, std::min<size_t>((size_t)ctx->ntau, ((size_t)8 << 30) / per_lag));
+    plan_lags(ctx, rs);
     exm_slot &sl = ctx->slot;
-    exm_ensure(ctx, sl.cnt, (size_t)rs.rc * EXM_NPAIR * (ctx->nm + 1) * sizeof(int));
-    const size_t pitch = (size_t)exm_desc_pitch((long long)ctx->nm * rs.nwalk);
-    exm_ensure(ctx, sl.desc, (size_t)rs.rc * pitch * sizeof(uint4));
-    exm_ensure(ctx, sl.tside, (size_t)rs.rc * pitch * sizeof(int32_t));
-    exm_ensure(ctx, sl.part, (size_t)(ctx->nn + 1) * ctx->ntau * ctx->nm * sizeof(double));
+    ensure_taps(ctx, sl, rs);
     EXM_CUDA(cudaMemsetAsync(sl.dev_err.p, 0, sizeof(unsigned), ctx->stream));
     ChunkInfo ci{0, ctx->nm, rs.nwalk, rs.use_sel, rs.lw};
     for (int r0 = 0; r0 < ctx->ntau; r0 += rs.rc) {
@@ -1463,13 +1477,11 @@ extern "C" int exm_node_values(exm_ctx *ctx, double *lamN_out)
         exm_run_taps(ctx, sl, ci, r0, rc, r0 == 0);
         exm_run_gather_planes(ctx, sl, ci, r0, rc);
     }
-    dbuf dl;
-    exm_alloc(ctx, dl, sizeof(double) * (size_t)(ctx->nn + 1) * ctx->nm);
-    exm_run_node_values(ctx, sl, (double *)dl.p);
+    exm_ensure(ctx, sl.lamN, (size_t)(ctx->nn + 1) * ctx->nm * sizeof(double));
+    exm_run_node_values(ctx, sl, 0, ctx->nm, (double *)sl.lamN.p);
     std::vector<double> h((size_t)(ctx->nn + 1) * ctx->nm);
-    EXM_CUDA(cudaMemcpyAsync(h.data(), dl.p, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, ctx->stream));
+    EXM_CUDA(cudaMemcpyAsync(h.data(), sl.lamN.p, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, ctx->stream));
     check_dev_err(ctx, sl);
-    exm_free(ctx, dl);
     for (int k = 0; k <= ctx->nn; ++k)
         for (int i = 0; i < ctx->nm; ++i) lamN_out[(size_t)k * ctx->nm + ctx->order[i]] = h[(size_t)k * ctx->nm + i];
     API_END(ctx)

@@ -56,7 +56,6 @@ struct dbuf {
 struct exm_slot {
     dbuf traj;      // float2 [2][nm][nt]: (ln|z|, arg z) of H then L
     dbuf trajlo;    // float [2][nm][nt]: ln|z| - float(ln|z|), filter precision 'fp64' only (0 for uploaded trajectories)
-    dbuf fft;       // double2 [2][nm][nt]: the padded rows and their transforms
     dbuf keys;      // uint32 [nm][nt]: selection scores as ordered integers
     dbuf picks;     // int32 [nm][S]: random ranks into the rest
     dbuf rej;       // int32 [1 + EXM_MAX_REJ]: rejected draw positions
@@ -64,15 +63,19 @@ struct exm_slot {
     dbuf hist;      // int32 histograms for the staging windows
     dbuf win;       // int32 window origins
     dbuf cnt;       // int32 [rc][48][nm+1]: taps per (lag, plane pair, template) -> offsets
-    dbuf desc;      // uint4 [rc][nm*nwalk]: tap descriptors sorted by (plane pair, template)
-    dbuf tside;     // int32 [rc][nm*nwalk]: time index of each descriptor (slow path)
-    dbuf part;      // double [nn+1][ntau][nm]: ln of the per-lag sums
+    dbuf desc;      // uint4 [rc][exm_desc_pitch]: tap descriptors sorted by (plane pair, template); before them, in the
+                    // same memory, double2 [2][nm][nt]: the filter's padded rows and their transforms
+    dbuf tside;     // int32 [rc][exm_desc_pitch]: time index of each descriptor (slow path)
+    dbuf part;      // double [nn+1][ntau][nparts][nm]: ln of the per-lag sums over parts of the plane pairs
+    dbuf lamN;      // double [nn+1][nm]: node values
     dbuf lnl;       // double [nm]
     dbuf lnb;       // double [1]
     dbuf dev_err;   // uint32 [1]
     dbuf hostin;    // pinned host staging (d_H, d_L)
     dbuf din;       // device copy of d_H, d_L complex128 and sig2
     int nwalk = 0, rc = 0;
+    int wb = 0, ng = 0;   // rows of the windows and groups per lane that the descriptors were built for (exm_gather_plan)
+    int nparts = 1;       // partial sums per (node, lag, template) in part (exm_gather_parts)
 };
 
 #define EXM_MAX_REJ 4096
@@ -120,8 +123,9 @@ struct exm_ctx {
     std::vector<float> tscale;   // per node: value = tscale[k] * stored element (1 for float32, bfloat16)
     dbuf d_tscale;               // float [nn]
     dbuf d_tau;         // int32 [ntau]
-    CUtensorMap tmap;   // 5-D map over T for the plane windows
+    CUtensorMap tmap;   // 5-D map over T for the plane windows of tmap_wb rows
     bool tmap_ok = false;
+    int tmap_wb = 0;
 
     // bank (original order)
     bool bank_ok = false;

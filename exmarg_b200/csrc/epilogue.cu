@@ -97,38 +97,69 @@ __global__ void k_distance_weights(const double *__restrict__ y, int nn1, int nm
     for (int j = 0; j < np_; ++j) lnW[(long long)idx[j] * nm + i] = log(w[j]);
 }
 
-// ln Lambda per template, and (optionally) the node values lamN (nn + 1, nm)
-__global__ void k_node_lse(const double *__restrict__ part, const double *__restrict__ lnW, const int *__restrict__ mlo,
-                           const int *__restrict__ mhi, const int *__restrict__ bnode, int nn, int ntau, int nm,
-                           int m_base, int nmc, int nt, double *__restrict__ lnl, double *__restrict__ lamN)
+// node values lamN (nn + 1, nm): the log-sum-exp over the lags' partial sums, minus ln n_time; -inf where the
+// template has no point.  A block is 32 templates of one node (row nn: the boundary points), its eight warps
+// share the partial sums: one thread per template over all nodes and lags was a chain of 9000 dependent
+// loads (0.86 ms a segment whatever the bank's size).
+__global__ void __launch_bounds__(256) k_node_values(const double *__restrict__ part, const int *__restrict__ mlo,
+                                                     const int *__restrict__ mhi, const int *__restrict__ bnode, int nn,
+                                                     int np, int nm, int m_base, int nmc, int nt,
+                                                     double *__restrict__ lamN)
 {
-    const int i = m_base + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m_base + nmc) return;
-    const double lnt = log((double)nt);
-    double M = -INFINITY, S = 0.0;
-    for (int k = 0; k <= nn; ++k) {
-        bool valid;
-        if (k < nn) valid = (i >= mlo[k] && i < mhi[k]);
-        else valid = bnode[i] >= 0;
-        double lam = -INFINITY;
-        if (valid) {
-            const double *pr = part + (long long)k * ntau * nm + i;
-            double mx = -INFINITY;
-            for (int r = 0; r < ntau; ++r) mx = fmax(mx, pr[(long long)r * nm]);
-            double tot = 0.0;
-            for (int r = 0; r < ntau; ++r) tot += exp(pr[(long long)r * nm] - mx);
-            lam = mx + log(tot) - lnt;
-        }
-        if (lamN) lamN[(long long)k * nm + i] = lam;
-        const double v = lnW[(long long)k * nm + i] + lam;
-        if (v > M) {
-            S = (M == -INFINITY) ? 1.0 : S * exp(M - v) + 1.0;
-            M = v;
-        } else if (v > -INFINITY) {
-            S += exp(v - M);
-        }
+    __shared__ double sm[8][32], ss[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i = m_base + blockIdx.x * 32 + lane, k = blockIdx.y;
+    const bool valid = i < m_base + nmc && (k < nn ? (i >= mlo[k] && i < mhi[k]) : bnode[i] >= 0);
+    const double *pr = part + (long long)k * np * nm + i;
+    double mx = -INFINITY;
+    if (valid)
+        for (int r = warp; r < np; r += 8) mx = fmax(mx, pr[(long long)r * nm]);
+    sm[warp][lane] = mx;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 8; ++q) mx = fmax(mx, sm[q][lane]);
+    double tot = 0.0;
+    if (valid)
+        for (int r = warp; r < np; r += 8) tot += exp(pr[(long long)r * nm] - mx);
+    ss[warp][lane] = tot;
+    __syncthreads();
+    if (warp == 0 && i < m_base + nmc) {
+        tot = 0.0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) tot += ss[q][lane];
+        lamN[(long long)k * nm + i] = valid ? mx + log(tot) - log((double)nt) : -INFINITY;
     }
-    lnl[i] = (M == -INFINITY) ? -INFINITY : M + log(S);
+}
+
+// ln Lambda per template: the log-sum-exp of lnW + lamN over the nodes and the boundary point; a block is 32
+// templates, its eight warps share the nodes
+__global__ void __launch_bounds__(256) k_node_lse(const double *__restrict__ lamN, const double *__restrict__ lnW, int nn1,
+                                                  int nm, int m_base, int nmc, double *__restrict__ lnl)
+{
+    __shared__ double sm[8][32], ss[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i = m_base + blockIdx.x * 32 + lane;
+    const bool on = i < m_base + nmc;
+    double M = -INFINITY, S = 0.0;
+    if (on)
+        for (int k = warp; k < nn1; k += 8) M = fmax(M, lnW[(long long)k * nm + i] + lamN[(long long)k * nm + i]);
+    sm[warp][lane] = M;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 8; ++q) M = fmax(M, sm[q][lane]);
+    if (on && M > -INFINITY)
+        for (int k = warp; k < nn1; k += 8) {
+            const double v = lnW[(long long)k * nm + i] + lamN[(long long)k * nm + i];
+            if (v > -INFINITY) S += exp(v - M);
+        }
+    ss[warp][lane] = S;
+    __syncthreads();
+    if (warp == 0 && on) {
+        S = 0.0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) S += ss[q][lane];
+        lnl[i] = (M == -INFINITY) ? -INFINITY : M + log(S);
+    }
 }
 
 // ln B = ln sum_i w_i exp(lnl_i) over the finite terms with w_i > 0 (one block)
@@ -164,21 +195,22 @@ __global__ void k_lnb(const double *__restrict__ lnl, const double *__restrict__
     }
 }
 
-void exm_run_node_lse(exm_ctx *ctx, exm_slot &sl, int m_base, int nmc)
+void exm_run_node_values(exm_ctx *ctx, exm_slot &sl, int m_base, int nmc, double *d_lamN)
 {
-    k_node_lse<<<(nmc + 127) / 128, 128, 0, ctx->stream>>>(
-        (const double *)sl.part.p, (const double *)ctx->d_lnW.p, (const int *)ctx->d_mlo.p, (const int *)ctx->d_mhi.p,
-        (const int *)ctx->d_bnode.p, ctx->nn, ctx->ntau, ctx->nm, m_base, nmc, ctx->nt, (double *)sl.lnl.p, nullptr);
+    k_node_values<<<dim3((nmc + 31) / 32, ctx->nn + 1), 256, 0, ctx->stream>>>(
+        (const double *)sl.part.p, (const int *)ctx->d_mlo.p, (const int *)ctx->d_mhi.p, (const int *)ctx->d_bnode.p,
+        ctx->nn, ctx->ntau * sl.nparts, ctx->nm, m_base, nmc, ctx->nt, d_lamN);
     EXM_CUDA(cudaGetLastError());
     ctx->launches += 1;
 }
 
-void exm_run_node_values(exm_ctx *ctx, exm_slot &sl, double *d_lamN)
+void exm_run_node_lse(exm_ctx *ctx, exm_slot &sl, int m_base, int nmc)
 {
-    k_node_lse<<<(ctx->nm + 127) / 128, 128, 0, ctx->stream>>>(
-        (const double *)sl.part.p, (const double *)ctx->d_lnW.p, (const int *)ctx->d_mlo.p, (const int *)ctx->d_mhi.p,
-        (const int *)ctx->d_bnode.p, ctx->nn, ctx->ntau, ctx->nm, 0, ctx->nm, ctx->nt, (double *)sl.lnl.p, d_lamN);
+    exm_run_node_values(ctx, sl, m_base, nmc, (double *)sl.lamN.p);
+    k_node_lse<<<(nmc + 31) / 32, 256, 0, ctx->stream>>>((const double *)sl.lamN.p, (const double *)ctx->d_lnW.p,
+                                                         ctx->nn + 1, ctx->nm, m_base, nmc, (double *)sl.lnl.p);
     EXM_CUDA(cudaGetLastError());
+    ctx->launches += 1;
 }
 
 void exm_run_lnb(exm_ctx *ctx, exm_slot &sl)

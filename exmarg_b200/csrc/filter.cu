@@ -68,7 +68,7 @@ void exm_run_filter(exm_ctx *ctx, exm_slot &sl, const float2 *dW, int nm)
     float2 *w = (float2 *)((char *)sl.din.p + (size_t)6 * nf * sizeof(double) + 4 * sizeof(uint64_t));
     k_weights<<<(2 * nf + 255) / 256, 256, 0, ctx->stream>>>((const double *)sl.din.p, nf, w);
     const long long total = 2LL * nm * nt;
-    double2 *z = (double2 *)sl.fft.p;
+    double2 *z = (double2 *)sl.desc.p;   // dead before the tap build writes descriptors there
     k_premul<<<(unsigned)((total + 255) / 256), 256, 0, ctx->stream>>>(dW, w, nm, nf, ctx->lo, nt, z);
     EXM_CUDA(cudaGetLastError());
     exm_fft_plan(ctx, 2 * nm);

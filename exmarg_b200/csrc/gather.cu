@@ -1,18 +1,28 @@
 // The table read of Eq. (C7) (exmarg/search/gather.py:32-107) on the B200.
 //
-// k_gather_planes (the pe_intrinsic path): one block per (node k, lag r, block of up
-// to 2048 templates).  The block walks the 48 phase-plane pairs (p, p+1) of the
-// node's lag slab T[k, r]; for each plane it stages, with one TMA copy, a window of
-// 80 beta rows x 160 Delta columns into shared memory (three slots: two planes in
-// use, one in flight).  The descriptors of the lag are sorted by (plane pair,
-// template), and each warp owns a contiguous range of templates, so for each pair a
-// warp reads one contiguous run of 16-byte descriptors, evaluates the bilinear x
-// linear interpolation from shared memory, and merges the log-sum-exp of each
-// template with warp shuffles into a per-template accumulator that only it writes.
-// Values are carried as (B, e) with B a stored float32 table value and e a small
-// float32 correction, so a tap of size ~1e3 keeps ~1e-7 absolute precision.  Taps
-// outside the window, and taps whose beta is clamped to the table, take an exact
-// float64 path that reads the table from global memory.
+// k_gather_planes (the pe_intrinsic path): one block per (lag r, template chunk, node k).  The block walks
+// the 48 phase-plane pairs (p, p+1) of the node's lag slab T[k, r]; for each plane it stages, with one TMA
+// copy, a window of 80-160 beta rows x 160 (16-bit tables: 192) Delta columns into shared memory (three
+// slots: two planes in use, one in flight).  The descriptors of the lag are sorted by (plane pair,
+// template) in groups of four taps of one template, and each warp owns a contiguous range of groups: it
+// evaluates the bilinear x linear interpolation of a lane's four taps from shared memory, takes their maximum and
+// adds their exponentials to the lane's running partial of that template, and merges partials across lanes with
+// warp shuffles into a per-template accumulator that only it writes.
+// A value is carried as (B, e) with B a stored float32 table value and e a small float32 correction up to its
+// exponential, so a tap of size ~1e3 keeps ~1e-7 absolute precision; a partial is (m, S), S exp(m), with m the
+// largest value.  Taps outside the window, and taps whose beta is clamped to the table, take an exact float64
+// path that reads the table from global memory.
+//
+// What bounds it (2048 templates x 53 nodes x 87 lags x 2048 times, 1.65e10 taps): shared-memory reads (eight a
+// tap, 69 % of the data pipe) and instruction issue (61 %) together; DRAM is at a tenth of its rate.  92.7 -> 65.3 ms:
+//  * four taps of one template per group: the bookkeeping of templates, the ranges and the running maximum are paid
+//    once for four taps (5.4 -> 2.9 warp instructions per tap); padding the runs to whole groups adds 3.8 % taps;
+//  * a row pitch of a multiple of the 32 banks, and taps ordered so that a step's lanes hit different banks
+//    (k_tap_order): 3.4 -> 2.4 cycles per read;
+//  * boundary points in blocks of their own, so the accumulators take 24 instead of 80 bytes a template and a block
+//    takes 1024 templates: every plane pair costs a block a fixed ~6 us of waits (68.0 at 704, 75.5 at 352);
+//  * a warp's first descriptors and end templates of the next pair loaded before it waits for that pair's planes.
+// 20 warps at 96 registers: 16 warps 68.5 ms (too few to cover the latencies), 24 and 28 spill (67.0, 80.4).
 //
 // k_gather_simple (the gather_cpu / gather_gpu contract, any table per slot): one
 // block per (row, lag), the reference's arithmetic in float64.
@@ -26,10 +36,6 @@
 extern __shared__ __align__(1024) unsigned char exm_gsm[];
 __device__ __forceinline__ float *gsm_f(unsigned off) { return (float *)(exm_gsm + off); }
 
-// one staged (node, lag, plane) window of element type TE: EXM_WB rows x TabElem<TE>::wd columns
-template <typename TE> __host__ __device__ constexpr int slot_elems() { return EXM_WB * TabElem<TE>::wd; }
-template <typename TE> __host__ __device__ constexpr unsigned slot_bytes() { return (unsigned)(slot_elems<TE>() * sizeof(TE)); }
-static_assert(slot_bytes<float>() % 128 == 0 && slot_bytes<__half>() % 128 == 0, "slots keep 128-byte alignment");
 #define EXM_WAIT_CYCLES (2000000000LL)   // about one second at 1.9 GHz
 #define EXM_TEST_WAIT_CYCLES (20000LL)   // the wait-expiry test's limit (no copy is ever in flight then)
 
@@ -46,14 +52,17 @@ struct PlaneArgs {
     unsigned *err;
     unsigned long long *stats;   // [0] slow-path taps, [1] boundary taps (may be null)
     long long tstride, per_lag;
-    int nn, ntau, nphif, nb, nd, ndp, nt, nmc, m_base, nm_total, r0, tch, nch;
-    float lw;
+    int nn, ntau, nphif, nb, nd, ndp, nt, nmc, nwalk, m_base, nm_total, r0, tch, nch;
+    int wb, ng, nparts;          // window rows, groups per lane and chunk, parts of the plane pairs
+    float lw, wr;                // log weight of a random draw, and its exponential
+    int nbn, nchb, tchb;         // boundary nodes, template chunks of each, templates of a chunk
+    int bn_k[EXM_MAX_NODES], bn_lo[EXM_MAX_NODES], bn_hi[EXM_MAX_NODES];   // ... and their templates
     double rph, rdb, rdd, offd;
     long long wait_cycles;       // limit of the pipeline's barrier waits (EXM_WAIT_CYCLES)
     int stage;                   // 1: stage the planes; 0 (the wait-expiry test): no copy is issued, so the
                                  // first wait runs out and the kernel returns its timeout status
     int cki[EXM_MAX_NODES];
-    float ckf[EXM_MAX_NODES];
+    unsigned ckf[EXM_MAX_NODES];  // fraction of a node's beta shift, 23-bit fixed point
     float tsc[EXM_MAX_NODES];    // per node: value = tsc * stored element
 };
 
@@ -101,41 +110,89 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, unsign
     }
 }
 
-// ------------------------------------------------------------------ log-sum-exp of (B, e) values
+// ------------------------------------------------------------------ log-sum-exp partials (m, S): S exp(m)
 
-__device__ __forceinline__ void lse_merge(float &B, float &E, float &S, float B2, float E2, float S2)
+#define EXM_L2E 1.4426950408889634f
+#define EXM_MNONE (-1e30f)   // the reference of an empty partial
+
+__device__ __forceinline__ float ex2_approx(float x)
 {
-    // (B, E, S) += (B2, E2, S2): the larger of the two values becomes the reference, without a branch
-    const float d = (B2 - B) + (E2 - E);
-    const bool up = d > 0.f;
-    const float e = __expf(-fabsf(d));
-    const float s_up = fmaf(S, e, S2), s_dn = fmaf(S2, e, S);
-    B = up ? B2 : B;
-    E = up ? E2 : E;
-    S = up ? s_up : s_dn;
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
 }
 
-// segmented reduction over lanes with equal id (ids non-decreasing along the lanes of a run);
-// afterwards the first lane of each run holds the run's total
-__device__ __forceinline__ bool seg_reduce(int id, float &B, float &E, float &S)
+__device__ __forceinline__ void ms_merge(float &m, float &S, float m2, float S2)
+{
+    // (m, S) += (m2, S2): the larger of the two becomes the reference, without a branch
+    const float d = m2 - m;
+    const float e = ex2_approx(-fabsf(d) * EXM_L2E);
+    S = d > 0.f ? fmaf(S, e, S2) : fmaf(S2, e, S);
+    m = fmaxf(m, m2);
+}
+
+// segmented reduction over lanes with equal id (ids non-decreasing along the lanes); afterwards the
+// first lane of each run holds the run's total.  The references first (a running maximum), then the sums
+// scaled to the run's reference: two shuffles and two operations a round instead of a merge.  Rounds end
+// when no run reaches further.
+__device__ __forceinline__ bool seg_reduce(int id, float &m, float &S)
 {
     const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int id2 = __shfl_down_sync(0xffffffffu, id, o);
-        const float B2 = __shfl_down_sync(0xffffffffu, B, o);
-        const float E2 = __shfl_down_sync(0xffffffffu, E, o);
-        const float S2 = __shfl_down_sync(0xffffffffu, S, o);
-        if (lane + o < 32 && id2 == id) lse_merge(B, E, S, B2, E2, S2);
-    }
     const int prev = __shfl_up_sync(0xffffffffu, id, 1);
-    return lane == 0 || prev != id;
+    const bool head = lane == 0 || prev != id;
+    const unsigned heads = __ballot_sync(0xffffffffu, head);
+    // lanes from here to the end of the lane's run, and the run's first lane
+    const unsigned above = heads & ~((2u << lane) - 1u);
+    const int left = (above ? __ffs(above) - 1 : 32) - lane;
+    const int first = 31 - __clz(heads & ((2u << lane) - 1u));
+    const int longest = __reduce_max_sync(0xffffffffu, left);
+    float M = m;
+    for (int o = 1; o < longest; o <<= 1) {
+        const float m2 = __shfl_down_sync(0xffffffffu, M, o);
+        if (o < left) M = fmaxf(M, m2);
+    }
+    M = __shfl_sync(0xffffffffu, M, first);
+    S *= ex2_approx((m - M) * EXM_L2E);
+    m = M;
+    for (int o = 1; o < longest; o <<= 1) {
+        const float S2 = __shfl_down_sync(0xffffffffu, S, o);
+        if (o < left) S += S2;
+    }
+    return head;
+}
+
+// two float32 operations in one instruction (planes p and p + 1 of a tap side by side)
+typedef unsigned long long f2_t;
+__device__ __forceinline__ f2_t f2_pack(float a, float b)
+{
+    f2_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f2_unpack(f2_t v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f2_t f2_sub(f2_t a, f2_t b)
+{
+    f2_t r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2_t f2_mul(f2_t a, f2_t b)
+{
+    f2_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2_t f2_fma(f2_t a, f2_t b, f2_t c)
+{
+    f2_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
 }
 
 // bilinear in (beta, Delta) on planes p and p+1 of the staged windows, linear in phase;
-// value = t00 + eps with t00 the stored value at (p, b0, d0).  16-bit elements are
-// interpolated as stored (float32 arithmetic) and the result scaled by the node's power-of-two
-// scale, which is exact.
+// value = B + E with B the stored value at (p, b0, d0).  16-bit elements are interpolated as
+// stored (float32 arithmetic) and the result scaled by the node's power-of-two scale, which is
+// exact.
 template <typename TE>
 __device__ __forceinline__ void interp_window(const TE *s0, const TE *s1, int o, float fbf, float fd, float w, float sc,
                                               float &B, float &E)
@@ -145,10 +202,20 @@ __device__ __forceinline__ void interp_window(const TE *s0, const TE *s1, int o,
     const float t10 = TabElem<TE>::cvt(s0[o + WD]), t11 = TabElem<TE>::cvt(s0[o + WD + 1]);
     const float u00 = TabElem<TE>::cvt(s1[o]), u01 = TabElem<TE>::cvt(s1[o + 1]);
     const float u10 = TabElem<TE>::cvt(s1[o + WD]), u11 = TabElem<TE>::cvt(s1[o + WD + 1]);
+#ifdef EXM_SCALAR
     const float a0 = t01 - t00, c0 = t10 - t00, e0 = (t11 - t10) - a0;
     const float eps0 = fmaf(fd, a0, fbf * fmaf(fd, e0, c0));
     const float a1 = u01 - u00, c1 = u10 - u00, e1 = (u11 - u10) - a1;
     const float eps1 = fmaf(fd, a1, fbf * fmaf(fd, e1, c1));
+#else
+    const f2_t p00 = f2_pack(t00, u00);
+    const f2_t a = f2_sub(f2_pack(t01, u01), p00), c = f2_sub(f2_pack(t10, u10), p00);
+    const f2_t e = f2_sub(f2_sub(f2_pack(t11, u11), f2_pack(t10, u10)), a);
+    const f2_t fd2 = f2_pack(fd, fd), fb2 = f2_pack(fbf, fbf);
+    const f2_t eps = f2_fma(fd2, a, f2_mul(fb2, f2_fma(fd2, e, c)));
+    float eps0, eps1;
+    f2_unpack(eps, eps0, eps1);
+#endif
     B = t00;
     E = fmaf(w, (u00 - t00) + (eps1 - eps0), eps0);
     if (!std::is_same<TE, float>::value) {
@@ -157,83 +224,69 @@ __device__ __forceinline__ void interp_window(const TE *s0, const TE *s1, int o,
     }
 }
 
-__device__ __forceinline__ void split_double(double v, float &B, float &E)
-{
-    B = (float)v;
-    E = (float)(v - (double)B);
-}
-
-// One run of tap descriptors (sorted by template) on the two staged planes of pair p.
-// Each lane takes 4 consecutive taps of a 128-tap chunk and merges equal-template taps in
-// registers; a template that lies inside one lane's taps is merged into its accumulator by
-// that lane, one that spans lanes is combined by a segmented shuffle reduction once per chunk.
+// One run of tap descriptors (sorted by template, in groups of EXM_GT taps of one template) on the
+// two staged planes of pair p.  Each lane takes ng consecutive groups of a chunk; a template that
+// lies inside one lane's groups is merged into its accumulator by that lane, one that spans lanes
+// is combined by a segmented shuffle reduction once per chunk.
 // byte offsets below are into exm_gsm
 struct RunCtx {
     const uint4 *descr;
     const int32_t *tsr;
     unsigned s0, s1;            // the staged windows of planes p and p + 1 (element type TE)
     float sc;                   // the node's scale (16-bit tables)
-    unsigned acc, accst;        // accumulator set of the run's templates (B at acc + 4 (t - lo); E, S at
-                                // + accst, + 2 accst)
-    unsigned bsh, bcf;          // boundary runs: per-template window-row shift (int; EXM_BSH_NONE for templates
-                                // whose boundary point is not this node) and beta fraction
+    unsigned acc, accst;        // accumulator set of the run's templates (m at acc + 4 t; S at + accst)
+    unsigned bsh, bcf;          // boundary blocks: per-template window offset (int; EXM_BSH_NONE for templates
+                                // whose boundary point is not this node) and beta fraction (23-bit fixed point)
+    int ng;                     // groups per lane and chunk
     int lo, m_base, n, k, r;
-    int sh;                     // window row of a tap = rb0 + carry + sh (regular runs)
-    int up, edge;               // fast path: row <= up, and not (row == edge with beta at the clamp)
-    float ckf, lw;
+    int sh;                     // window offset of a tap = its o0 + sh (+ a row when the beta fractions carry)
+    unsigned lim;               // the taps the windows serve have offsets below lim
+    unsigned ckf;               // the node's beta fraction, 23-bit fixed point
+    float wr, lw;               // weight of a random draw and its logarithm
+    int beg, end;               // the warp's sorted positions (whole groups)
     int tF, tL;                 // the templates at the two ends of this warp's taps (may be shared with
-    unsigned eF, eL;            // neighbouring warps): their partials go to this warp's edge slots (B, E, S)
+    unsigned eF, eL;            // neighbouring warps): their partials go to this warp's edge slots (m, S)
     unsigned q, qn;             // this warp's queue of exact-path taps for the pair (int2 entries) and its count
+    // the lane's next group of descriptors: whether it lies in [beg, end), its first position, its address,
+    // its index in the chunk
+    uint4 nx[EXM_GT];
+    bool in;
+    int jl, gn;
+    const uint4 *pn;
 };
 
-__device__ __forceinline__ void acc_merge(const RunCtx &c, int tr, float B, float E, float S)
+// load the lane's next group and step to the one after
+__device__ __forceinline__ void next_group(RunCtx &c)
+{
+    c.in = c.jl >= c.beg && c.jl < c.end;
+#pragma unroll
+    for (int u = 0; u < EXM_GT; ++u) c.nx[u] = c.in ? __ldg(c.pn + 32 * u) : make_uint4(0u, 0u, 0u, EXM_DESC_PAD);
+    c.pn += 32 * EXM_GT;
+    c.jl += EXM_GT;
+    if (++c.gn == c.ng) {   // on to the next chunk
+        c.gn = 0;
+        c.jl += EXM_GT * 31 * c.ng;
+    }
+}
+
+__device__ __forceinline__ void acc_merge(const RunCtx &c, int tr, float m, float S)
 {
     const bool f = tr == c.tF, l = tr == c.tL;
     const unsigned off = f ? c.eF : (l ? c.eL : c.acc + 4u * (unsigned)tr);
     const unsigned st = (f || l) ? 4u : c.accst;
-    float *pB = gsm_f(off), *pE = gsm_f(off + st), *pS = gsm_f(off + 2 * st);
-    float b = *pB, e = *pE, s = *pS;
-    lse_merge(b, e, s, B, E, S);
-    *pB = b;
-    *pE = e;
-    *pS = s;
+    float *pm = gsm_f(off), *pS = gsm_f(off + st);
+    float m1 = *pm, S1 = *pS;
+    ms_merge(m1, S1, m, S);
+    *pm = m1;
+    *pS = S1;
 }
 
-#define TPL EXM_TPL   // consecutive taps per lane (in groups of GRP); a warp chunk is EXM_DCH taps
-#ifndef EXM_GUNROLL
-#define EXM_GUNROLL 2
-#endif
-constexpr int kGroupUnroll = EXM_GUNROLL;   // tap groups of a chunk unrolled in the lane loop
-#define EXM_SLOWQ 8   // exact-path taps a consumer warp queues per plane pair for the producer
-#define EXM_BSH_NONE (-(1 << 28))   // bsh entry of a template whose boundary point is another node
-
-
-// the lane-local running segmented merge of one value (taps arrive sorted by template)
-__device__ __forceinline__ void lane_merge(const RunCtx &c, int t, float vB, float vE, float wt, int &cT, float &cB,
-                                           float &cE, float &cS, int &fT, float &fB, float &fE, float &fS)
-{
-    // branch-free except for the rare template that opens and closes inside one lane
-    const bool nw = t != cT;
-    const bool close = nw && cT >= 0;      // cT closes here
-    const bool toF = close && fT < 0;      // ... as the lane's first closed partial
-    if (close && !toF) acc_merge(c, cT, cB, cE, cS);
-    fT = toF ? cT : fT;
-    fB = toF ? cB : fB;
-    fE = toF ? cE : fE;
-    fS = toF ? cS : fS;
-    cT = nw ? t : cT;                      // a new template starts from an empty partial
-    cB = nw ? -1e30f : cB;
-    cE = nw ? 0.f : cE;
-    cS = nw ? 0.f : cS;
-    lse_merge(cB, cE, cS, vB, vE, wt);
-}
+#define EXM_SLOWQ 12   // exact-path taps a consumer warp queues per plane pair for the producer
+#define EXM_BSH_NONE (1 << 29)   // bsh entry of a template whose boundary point is another node
 
 // the exact float64 value of a tap outside the staged window (rare)
-#ifndef EXM_SLOW_INLINE
-#define EXM_SLOW_INLINE __forceinline__
-#endif
 template <bool BND, typename TE>
-__device__ EXM_SLOW_INLINE double slow_tap(const PlaneArgs &a, int il, int tm, int k, int r, int m_base, float sc)
+__device__ __forceinline__ double slow_tap(const PlaneArgs &a, int il, int tm, int k, int r, int m_base, float sc)
 {
     const int nt = a.nt;
     const int tau0 = ((a.tau[r] % nt) + nt) % nt;
@@ -248,236 +301,263 @@ __device__ EXM_SLOW_INLINE double slow_tap(const PlaneArgs &a, int il, int tm, i
                             a.rdd, a.offd);
 }
 
-// GRP taps: decode, window interpolation for all of them (no branch between the shared loads),
-// the exact float64 value for the rare taps outside the window, then the merges
-template <bool BND, int GRP, typename TE>
-__device__ __forceinline__ void tap_group(const PlaneArgs &a, const RunCtx &c, const uint4 *q, int j, int pj, int beg,
-                                          int end, int &cT, float &cB, float &cE, float &cS, int &fT, float &fB,
-                                          float &fE, float &fS, unsigned &n_slow)
+// a float64 value as a partial: its float32 rounding and the exponential of the rest
+__device__ __forceinline__ void split_double(double v, float &m, float &S)
 {
-    // j: sorted position of the group's first tap (taps j .. j + GRP - 1 of this lane);
-    // pj: its storage index (tap u of the group at pj + 32 u)
-    int t[GRP], o[GRP];
-    bool fast[GRP];
-    float fbf[GRP], fd[GRP], w[GRP], lwv[GRP], vB[GRP], vE[GRP];
-#pragma unroll
-    for (int u = 0; u < GRP; ++u) {
-        int tt = (j + u >= beg && j + u < end) ? (int)(q[u].w >> 19) + c.m_base - c.lo : -1;
-        if (tt >= c.n) {   // outside the block's templates: report and skip
-            atomicOr(a.err, EXM_DEVERR_BOUNDS);
-            tt = -1;
-        }
-        // boundary runs: the template's window-row shift, EXM_BSH_NONE unless its boundary point is this node
-        int bs = 0;
-        if (BND) {
-            bs = tt >= 0 ? ((const int *)gsm_f(c.bsh))[tt] : EXM_BSH_NONE;
-            if (bs == EXM_BSH_NONE) tt = -1;
-        }
-        t[u] = tt;
-        const int ts = tt >= 0 ? tt : 0;
-        const float fb = __uint_as_float(q[u].x);
-        fd[u] = __uint_as_float(q[u].y);
-        w[u] = __uint_as_float(q[u].z & 0x7FFFFFFFu);
-        lwv[u] = (q[u].z >> 31) ? c.lw : 0.f;
-        const int rd = (int)((q[u].w >> 11) & 0xFFu);      // window column (255: outside)
-        const int rb0 = ((int)(q[u].w << 21)) >> 21;        // beta-hat row from the window origin
-        const float sfr = fb + (BND ? gsm_f(c.bcf)[ts] : c.ckf);
-        const int cy = sfr >= 1.f;
-        fbf[u] = cy ? sfr - 1.f : sfr;
-        const int rb = rb0 + cy + (BND ? bs : c.sh);   // this node's window row
-        constexpr int WD = TabElem<TE>::wd;
-        fast[u] = (unsigned)rb <= (unsigned)c.up && rd <= WD - 2 && !(rb == c.edge && fbf[u] > 0.999999f);
-        o[u] = fast[u] ? rb * WD + rd : 0;
-    }
-#pragma unroll
-    for (int u = 0; u < GRP; ++u)
-        interp_window<TE>((const TE *)(exm_gsm + c.s0), (const TE *)(exm_gsm + c.s1), o[u], fbf[u], fd[u], w[u], c.sc,
-                          vB[u], vE[u]);
-    float wt[GRP];
-#pragma unroll
-    for (int u = 0; u < GRP; ++u) {
-        const bool sl = t[u] >= 0 && !fast[u];
-        wt[u] = t[u] >= 0 ? 1.f : 0.f;
-        if (__any_sync(0xffffffffu, sl)) {
-            // exact-path taps go to the warp's queue: the producer computes them 32 at a time instead
-            // of stalling the warp on one lane's float64 path; a full queue computes them here
-            const int lane = threadIdx.x & 31;
-            const unsigned m = __ballot_sync(0xffffffffu, sl);
-            int *qn = (int *)(exm_gsm + c.qn);
-            const int n0 = *qn;
-            const int pos = n0 + __popc(m & ((1u << lane) - 1u));
-            __syncwarp();
-            if (sl) {
-                ++n_slow;
-                if (pos < EXM_SLOWQ) {
-                    ((int2 *)(exm_gsm + c.q))[pos] =
-                        make_int2(pj + 32 * u, (int)(q[u].w >> 19) | (BND ? 1 << 30 : 0) | (int)((q[u].z >> 31) << 29));
-                    vB[u] = -1e30f;
-                    vE[u] = 0.f;
-                    wt[u] = 0.f;
-                    lwv[u] = 0.f;
-                } else {
-                    const double v =
-                        slow_tap<BND, TE>(a, (int)(q[u].w >> 19), c.tsr[pj + 32 * u], c.k, c.r, c.m_base, c.sc);
-                    split_double(v, vB[u], vE[u]);
-                }
-            }
-            if (lane == 0) *qn = min(EXM_SLOWQ, n0 + __popc(m));
-            __syncwarp();
-        }
-    }
-#pragma unroll
-    for (int u = 0; u < GRP; ++u)
-        lane_merge(c, t[u], vB[u], vE[u] + lwv[u], wt[u], cT, cB, cE, cS, fT, fB, fE, fS);
+    m = (float)v;
+    S = ex2_approx((float)(v - (double)m) * EXM_L2E);
 }
 
-template <bool BND, int GRP, typename TE>
-__device__ void process_run(const PlaneArgs &a, const RunCtx &c, int beg, int end, unsigned &n_slow)
+// the taps of a group that the windows do not serve (storage index pj + 32 u): queued for the producer, which
+// computes them 32 at a time instead of stalling the warp on one lane's float64 path; those a full queue
+// cannot take are computed here and merged into the lane's running partial
+template <bool BND, typename TE>
+__device__ __forceinline__ void slow_group(const PlaneArgs &a, const RunCtx &c, int pj, int t, int sh, unsigned ckf,
+                                           float &m, float &S, unsigned &n_slow)
 {
-    // the warp's sorted positions [beg, end), walked in whole chunks of EXM_DCH (positions outside
-    // [beg, end) masked); lane l takes the chunk's positions l*TPL + i, stored at i*32 + l
     const int lane = threadIdx.x & 31;
-    const int jstart = beg & ~(EXM_DCH - 1);
-    uint4 qa[GRP];
-#pragma unroll
-    for (int u = 0; u < GRP; ++u) {
-        const int jl = jstart + TPL * lane + u;
-        qa[u] = (jl >= beg && jl < end) ? __ldg(c.descr + jstart + 32 * u + lane) : make_uint4(0u, 0u, 0u, 0u);
-    }
-    for (int j0 = jstart; j0 < end; j0 += EXM_DCH) {
-        const int jb = j0 + TPL * lane;
-        int cT = -1, fT = -1;
-        float cB = -1e30f, cE = 0.f, cS = 0.f, fB = -1e30f, fE = 0.f, fS = 0.f;
-#pragma unroll(kGroupUnroll)
-        for (int g = 0; g < TPL / GRP; ++g) {
-            uint4 cur[GRP];
-#pragma unroll
-            for (int u = 0; u < GRP; ++u) cur[u] = qa[u];
-            // the next group of descriptors (this lane's next group, or the next chunk's first)
-            const bool same = g + 1 < TPL / GRP;
-            const int jn0 = same ? j0 : j0 + EXM_DCH;
-            const int gn = same ? (g + 1) * GRP : 0;
-            if (same || j0 + EXM_DCH < end) {
-#pragma unroll
-                for (int u = 0; u < GRP; ++u) {
-                    const int jl = jn0 + TPL * lane + gn + u;
-                    qa[u] = (jl >= beg && jl < end) ? __ldg(c.descr + jn0 + 32 * (gn + u) + lane)
-                                                    : make_uint4(0u, 0u, 0u, 0u);
-                }
-            }
-            tap_group<BND, GRP, TE>(a, c, cur, jb + g * GRP, j0 + 32 * g * GRP + lane, beg, end, cT, cB, cE, cS, fT,
-                                    fB, fE, fS, n_slow);
+    int *qn = (int *)(exm_gsm + c.qn);
+#pragma unroll 1
+    for (int u = 0; u < EXM_GT; ++u, pj += 32) {
+        bool sl = false;
+        uint4 q = make_uint4(0u, 0u, 0u, EXM_DESC_PAD);
+        if (t >= 0) {
+            q = __ldg(c.descr + pj);
+            const int o = ((int)q.w >> 13) + sh + (int)((q.x + ckf) >> 23) * TabElem<TE>::wd;
+            sl = (unsigned)o >= c.lim && (int)q.w >= EXM_DESC_REAL;
         }
-        // the first closed template of lane l + 1 continues lane l's last one, or is lane l + 1's alone
-        const int nT = __shfl_down_sync(0xffffffffu, fT, 1);
-        const float nB = __shfl_down_sync(0xffffffffu, fB, 1);
-        const float nE = __shfl_down_sync(0xffffffffu, fE, 1);
-        const float nS = __shfl_down_sync(0xffffffffu, fS, 1);
-        const int pT = __shfl_up_sync(0xffffffffu, cT, 1);
-        if (lane < 31 && nT >= 0 && nT == cT) lse_merge(cB, cE, cS, nB, nE, nS);
-        if (fT >= 0 && !(lane > 0 && pT == fT)) acc_merge(c, fT, fB, fE, fS);
-        // last templates: runs across consecutive lanes
-        const bool head = seg_reduce(cT >= 0 ? cT : -2 - lane, cB, cE, cS);
-        if (head && cT >= 0) acc_merge(c, cT, cB, cE, cS);
+        const unsigned bal = __ballot_sync(0xffffffffu, sl);
+        if (!bal) continue;
+        const int n0 = *qn;
+        const int pos = n0 + __popc(bal & ((1u << lane) - 1u));
+        __syncwarp();
+        if (sl) {
+            ++n_slow;
+            const int il = (int)(q.w & 0x1FFFu);
+            if (pos < EXM_SLOWQ) {
+                ((int2 *)(exm_gsm + c.q))[pos] = make_int2(pj, il | (int)((q.z >> 31) << 29));
+            } else {
+                double v = slow_tap<BND, TE>(a, il, c.tsr[pj], c.k, c.r, c.m_base, c.sc);
+                if (q.z >> 31) v += (double)c.lw;
+                float m2, S2;
+                split_double(v, m2, S2);
+                ms_merge(m, S, m2, S2);
+            }
+        }
+        if (lane == 0) *qn = min(EXM_SLOWQ, n0 + __popc(bal));
+        __syncwarp();
     }
 }
 
-// the template of the descriptor at sorted position j (block-local), or -1
+#define EXM_EDGE_F 6   // floats of a warp's edge slots: (m, S, template) of its first and of its last template
+
+// the template of the descriptor at sorted position j (block-local)
 __device__ __forceinline__ int desc_template(const RunCtx &c, int j)
 {
-    return (int)(__ldg(&c.descr[exm_desc_phys(j)].w) >> 19) + c.m_base - c.lo;
+    return (int)(__ldg(&c.descr[exm_desc_phys(j, c.ng)].w) & 0x1FFFu) + c.m_base - c.lo;
 }
 
-// fold the warps' edge partials into the accumulators: one warp, lane w holding warp w's first (F)
-// and last (L) partials; templates ascend along the warps, so this is the lane-level merge again
-__device__ __forceinline__ void fold_edges(float *edge, int nw, float *aB, float *aE, float *aS, int n)
-{
-    const int lane = threadIdx.x & 31;
-    float fB = -1e30f, fE = 0.f, fS = 0.f, cB = -1e30f, cE = 0.f, cS = 0.f;
-    int fT = -1, cT = -1;
-    if (lane < nw) {
-        const float *e = edge + 8 * lane;
-        fT = __float_as_int(e[3]);
-        fB = e[0];
-        fE = e[1];
-        fS = e[2];
-        cT = __float_as_int(e[7]);
-        cB = e[4];
-        cE = e[5];
-        cS = e[6];
-        if (!(fT >= 0 && fT < n && fS > 0.f)) fT = -1;
-        if (!(cT >= 0 && cT < n)) cT = -1;
-    }
-    const int nT = __shfl_down_sync(0xffffffffu, fT, 1);
-    const float nB = __shfl_down_sync(0xffffffffu, fB, 1);
-    const float nE = __shfl_down_sync(0xffffffffu, fE, 1);
-    const float nS = __shfl_down_sync(0xffffffffu, fS, 1);
-    const int pT = __shfl_up_sync(0xffffffffu, cT, 1);
-    if (lane < 31 && nT >= 0 && nT == cT) lse_merge(cB, cE, cS, nB, nE, nS);
-    if (fT >= 0 && !(lane > 0 && pT == fT)) {
-        float b = aB[fT], x = aE[fT], q = aS[fT];
-        lse_merge(b, x, q, fB, fE, fS);
-        aB[fT] = b;
-        aE[fT] = x;
-        aS[fT] = q;
-    }
-    const bool head = seg_reduce(cT >= 0 ? cT : -2 - lane, cB, cE, cS);
-    if (head && cT >= 0 && cS > 0.f) {
-        float b = aB[cT], x = aE[cT], q = aS[cT];
-        lse_merge(b, x, q, cB, cE, cS);
-        aB[cT] = b;
-        aE[cT] = x;
-        aS[cT] = q;
-    }
-}
-
-// this warp's equal share [w0, w1) of the run [beg, end), with its edge templates and slots
-template <bool BND, int GRP, int NW, typename TE>
-__device__ __forceinline__ void warp_share(const PlaneArgs &a, RunCtx &c, int beg, int end, unsigned edge, int pair,
-                                           unsigned &n_slow)
+// this warp's share [c.beg, c.end) of the pair's run [beg, end): whole storage chunks per warp, as evenly as
+// they divide (the first and last may be partial), and the loads of its first group and of its end
+// templates, which are in flight while the warp waits for the pair's planes.
+// The warps with work are a prefix: the edge fold merges equal templates of neighbouring lanes only, so
+// an empty warp between two that share a template would let both update its accumulator at once.  When
+// every warp has a chunk, the rem warps that take one more are a cyclic window that moves by rem with the
+// pair, so that no warp takes the extra chunk at every pair: a warp runs at most one pair ahead, so with a
+// fixed prefix the others would wait at every pair.
+template <int NW>
+__device__ __forceinline__ void open_share(RunCtx &c, int beg, int end, int pair)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // whole storage chunks per warp, as evenly as they divide (the first and last may be partial).
-    // The warps with work are a prefix: the edge fold merges equal templates of neighbouring lanes
-    // only, so an empty warp between two that share a template would let both update its
-    // accumulator at once.  When every warp has a chunk, the rem warps that take one more are a
-    // cyclic window that moves by rem with the pair, so that no warp takes the extra chunk at every
-    // pair: a warp runs at most one pair ahead, so with a fixed prefix the others would wait at every pair.
-    const int cb = beg / EXM_DCH, nc = (end + EXM_DCH - 1) / EXM_DCH - cb;
+    const int ch = EXM_GT * 32 * c.ng;
+    const int cb = beg / ch, nc = (end + ch - 1) / ch - cb;
     const int q = nc / NW, rem = nc % NW;
     const int s = q > 0 ? (pair * rem) % NW : 0, se = s + rem;
     const int before = max(0, min(warp, se) - s) + max(0, min(warp, se - NW));   // extra chunks of warps < warp
     const int c0 = cb + warp * q + before, c1 = c0 + q + ((warp - s + NW) % NW < rem ? 1 : 0);
-    const int w0 = max(beg, c0 * EXM_DCH), w1 = min(end, c1 * EXM_DCH);
-    const unsigned eo = edge + 32u * warp;   // 8 floats per warp
-    float *e = gsm_f(eo);
-    int tF = -1, tL = -1;
-    if (w0 < w1) {
-        tF = desc_template(c, w0);
-        tL = desc_template(c, w1 - 1);
+    c.beg = max(beg, c0 * ch);
+    c.end = min(end, c1 * ch);
+    c.tF = c.tL = -1;
+    if (c.beg < c.end) {
+        const int jstart = c.beg & ~(ch - 1);
+        c.gn = 0;
+        c.jl = jstart + EXM_GT * c.ng * lane;
+        c.pn = c.descr + jstart + lane;
+        next_group(c);
+        c.tF = desc_template(c, c.beg);
+        c.tL = desc_template(c, c.end - 1);
     }
-    if (lane == 0) {
-        e[0] = -1e30f;
+}
+
+// the warp's edge slots of the pair, empty: one template only takes the L slot
+__device__ __forceinline__ void open_edge(RunCtx &c, unsigned eo)
+{
+    if (c.tF == c.tL) c.tF = -1;
+    c.eF = eo;
+    c.eL = eo + 12u;
+    if ((threadIdx.x & 31) == 0) {
+        float *e = gsm_f(eo);
+        e[0] = EXM_MNONE;
         e[1] = 0.f;
-        e[2] = 0.f;
-        e[3] = __int_as_float(tF == tL ? -1 : tF);
-        e[4] = -1e30f;
-        e[5] = 0.f;
-        e[6] = 0.f;
-        e[7] = __int_as_float(tL);
+        e[2] = __int_as_float(c.tF);
+        e[3] = EXM_MNONE;
+        e[4] = 0.f;
+        e[5] = __int_as_float(c.tL);
     }
     __syncwarp();
-    c.tF = (tF == tL) ? -1 : tF;   // one template only: the L slot takes it all
-    c.tL = tL;
-    c.eF = eo;
-    c.eL = eo + 16u;
-    if (w0 < w1) process_run<BND, GRP, TE>(a, c, w0, w1, n_slow);
+}
+
+template <bool BND, int PF, typename TE>
+__device__ __forceinline__ void process_run(const PlaneArgs &a, RunCtx &c, unsigned &n_slow)
+{
+    // the warp's positions walked in chunks of 128 ng; lane l takes the chunk's groups l ng + g, tap u of it
+    // stored at (g EXM_GT + u) 32 + l
+    constexpr int WD = TabElem<TE>::wd;
+    const int lane = threadIdx.x & 31;
+    const int ng = c.ng, ch = EXM_GT * 32 * ng, end = c.end;
+    for (int j0 = c.beg & ~(ch - 1); j0 < end; j0 += ch) {
+        int cT = -1, fT = -1;
+        float cm = EXM_MNONE, cS = 0.f, fm = EXM_MNONE, fS = 0.f;
+#pragma unroll 1
+        for (int g = 0; g < ng; ++g) {
+            // the group's template (-1: nothing to do) and the window shift of its taps
+            int t = (int)(c.nx[0].w & 0x1FFFu) + c.m_base - c.lo;
+            if (!c.in) t = -1;
+            if (t >= c.n) {   // outside the block's templates: report and skip
+                atomicOr(a.err, EXM_DEVERR_BOUNDS);
+                t = -1;
+            }
+            int sh = c.sh;
+            unsigned ckf = c.ckf;
+            if (BND) {
+                sh = EXM_BSH_NONE;
+                ckf = 0u;
+                if (t >= 0) {
+                    sh = ((const int *)gsm_f(c.bsh))[t];
+                    ckf = ((const unsigned *)gsm_f(c.bcf))[t];
+                }
+                if (sh == EXM_BSH_NONE) t = -1;
+            }
+            // window offset, beta and Delta fractions, plane weight and draw weight of the four taps
+            int o[EXM_GT];
+            float fb[EXM_GT], fd[EXM_GT], w[EXM_GT], wt[EXM_GT];
+            bool fast[EXM_GT];
+            bool sl = false;
+#pragma unroll
+            for (int u = 0; u < EXM_GT; ++u) {
+                const unsigned f = c.nx[u].x + ckf;
+                const int ou = ((int)c.nx[u].w >> 13) + sh + (int)(f >> 23) * WD;
+                fast[u] = (unsigned)ou < c.lim;
+                sl = sl || (!fast[u] && (int)c.nx[u].w >= EXM_DESC_REAL);
+                o[u] = fast[u] ? ou : lane;
+                fb[u] = __uint_as_float((f & 0x7FFFFFu) | 0x3F800000u) - 1.f;
+                fd[u] = __uint_as_float(c.nx[u].y);
+                w[u] = __uint_as_float(c.nx[u].z);
+                wt[u] = w[u] < 0.f ? c.wr : 1.f;
+            }
+            next_group(c);
+            // close the running template where another one begins
+            const bool nw = t != cT;
+            const bool close = nw && cT >= 0;
+            const bool toF = close && fT < 0;      // ... as the lane's first closed partial
+            if (close && !toF) acc_merge(c, cT, cm, cS);
+            fT = toF ? cT : fT;
+            fm = toF ? cm : fm;
+            fS = toF ? cS : fS;
+            cT = t;
+            cm = nw ? EXM_MNONE : cm;
+            cS = nw ? 0.f : cS;
+            float B[EXM_GT], E[EXM_GT];
+            float m = cm;
+#pragma unroll
+            for (int u = 0; u < EXM_GT; ++u) {
+                interp_window<TE>((const TE *)(exm_gsm + c.s0), (const TE *)(exm_gsm + c.s1), o[u], fb[u], fd[u],
+                                  fabsf(w[u]), c.sc, B[u], E[u]);
+                const float v = B[u] + E[u];
+                if (fast[u]) m = fmaxf(m, v);
+                if (PF == 1 && u == 1) __syncwarp();   // two taps' window reads in flight, for shapes with few registers
+            }
+            float S = cS * ex2_approx((cm - m) * EXM_L2E);
+#pragma unroll
+            for (int u = 0; u < EXM_GT; ++u) {
+                const float x = ex2_approx(((B[u] - m) + E[u]) * EXM_L2E);
+                if (fast[u]) S = fmaf(x, wt[u], S);
+            }
+            cm = m;
+            cS = S;
+            if (__any_sync(0xffffffffu, sl && t >= 0))
+                slow_group<BND, TE>(a, c, j0 + 32 * EXM_GT * g + lane, t, sh, ckf, cm, cS, n_slow);
+        }
+        // the first closed template of lane l + 1 continues lane l's last one, or is lane l + 1's alone
+        const int nT = __shfl_down_sync(0xffffffffu, fT, 1);
+        const float nm = __shfl_down_sync(0xffffffffu, fm, 1);
+        const float nS = __shfl_down_sync(0xffffffffu, fS, 1);
+        const int pT = __shfl_up_sync(0xffffffffu, cT, 1);
+        if (lane < 31 && nT >= 0 && nT == cT) ms_merge(cm, cS, nm, nS);
+        if (fT >= 0 && !(lane > 0 && pT == fT)) acc_merge(c, fT, fm, fS);
+        __syncwarp();
+        // last templates: runs across consecutive lanes
+        const bool head = seg_reduce(cT >= 0 ? cT : -2 - lane, cm, cS);
+        if (head && cT >= 0) acc_merge(c, cT, cm, cS);
+        __syncwarp();
+    }
+}
+
+// fold the warps' edge partials into the accumulators: one warp, lane w holding warp w's first (F)
+// and last (L) partials; templates ascend along the warps, so this is the lane-level merge again
+__device__ __forceinline__ void fold_edges(float *edge, int nw, float *am, float *aS, int n)
+{
+    const int lane = threadIdx.x & 31;
+    float fm = EXM_MNONE, fS = 0.f, cm = EXM_MNONE, cS = 0.f;
+    int fT = -1, cT = -1;
+    if (lane < nw) {
+        const float *e = edge + EXM_EDGE_F * lane;
+        fm = e[0];
+        fS = e[1];
+        fT = __float_as_int(e[2]);
+        cm = e[3];
+        cS = e[4];
+        cT = __float_as_int(e[5]);
+        if (!(fT >= 0 && fT < n && fS > 0.f)) fT = -1;
+        if (!(cT >= 0 && cT < n)) cT = -1;
+    }
+    const int nT = __shfl_down_sync(0xffffffffu, fT, 1);
+    const float nm = __shfl_down_sync(0xffffffffu, fm, 1);
+    const float nS = __shfl_down_sync(0xffffffffu, fS, 1);
+    const int pT = __shfl_up_sync(0xffffffffu, cT, 1);
+    if (lane < 31 && nT >= 0 && nT == cT) ms_merge(cm, cS, nm, nS);
+    if (fT >= 0 && !(lane > 0 && pT == fT)) {
+        float m = am[fT], S = aS[fT];
+        ms_merge(m, S, fm, fS);
+        am[fT] = m;
+        aS[fT] = S;
+    }
+    __syncwarp();
+    const bool head = seg_reduce(cT >= 0 ? cT : -2 - lane, cm, cS);
+    if (head && cT >= 0 && cS > 0.f) {
+        float m = am[cT], S = aS[cT];
+        ms_merge(m, S, cm, cS);
+        am[cT] = m;
+        aS[cT] = S;
+    }
 }
 
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar)
 {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+
+// shared memory of the plane gather after the three window slots, in bytes from the slots' end: barriers;
+// the accumulators, three sets of 2 x tch floats (m, S): pairs of parity 0 / 1, edges and exact-path taps
+// (producer) -- a boundary block has fewer templates, with bcf and bsh after its sets; the edge slots [pair
+// parity][EXM_EDGE_F floats per consumer warp]; exact-path queues [pair mod 3][consumer warp]: counts, then
+// EXM_SLOWQ int2 entries (storage index of the tap; template | random flag << 29)
+#define EXM_ACC_F 6    // floats per template: three sets of (m, S)
+#define EXM_ACCB_F 8   // ... of a boundary block: and bcf, bsh
+#define EXM_EDGE_B (4 * 2 * EXM_EDGE_F * 32)
+#define EXM_QCNT_B (4 * 3 * 32)
+#define EXM_QENT_B (8 * 3 * 32 * EXM_SLOWQ)
+#define EXM_GATHER_FIXED_B (64 + EXM_EDGE_B + EXM_QCNT_B + EXM_QENT_B)
 
 // Warp NW - 1 is the producer: it stages the planes with TMA and, once every consumer warp has
 // arrived on the pair's "done" barrier, folds that pair's edge partials and refills the slot of
@@ -486,71 +566,75 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar)
 // only after pair p is done everywhere).  So at most two consecutive pairs are in flight, and the
 // consumers' accumulators alternate with the pair's parity (two warps in different pairs never
 // share a word), while the producer folds edges into a third set of its own.
-template <int NW, int GRP, typename TE>
+template <int NW, int PF, typename TE>
 __global__ void __launch_bounds__(NW * 32, 1) k_gather_planes(const __grid_constant__ CUtensorMap tmap,
                                                                 const __grid_constant__ PlaneArgs a)
 {
     constexpr int NC = NW - 1;   // consumer warps
-    constexpr int SLOT = slot_elems<TE>();
-    constexpr unsigned SLOT_B = slot_bytes<TE>();
+    const int SLOT = a.wb * TabElem<TE>::wd;
+    const unsigned SLOT_B = (unsigned)SLOT * (unsigned)sizeof(TE);
     unsigned char *smem = exm_gsm;
     TE *win = (TE *)smem;
     uint64_t *full = (uint64_t *)(smem + 3 * SLOT_B);   // [3] plane staged in slot s
     uint64_t *done = full + 3;                          // [2] every consumer is done with a pair (parity)
-    const int tch = a.tch;
-    // accumulator sets of 3 x tch floats (B, E, S): regular pairs of parity 0 / 1, regular edges
-    // (producer), boundary pairs of parity 0 / 1, boundary edges; then bcf, bsh; then the edge
-    // slots [pair parity][regular, boundary][8 floats per consumer warp: F and L partials + ids]
-    const unsigned acc_o = 3 * SLOT_B + 64;
-    float *acc = gsm_f(acc_o);
-    float *bcf = acc + 18 * tch;
-    int *bsh = (int *)(bcf + tch);
-    const unsigned bcf_o = acc_o + 4u * 18u * tch, bsh_o = bcf_o + 4u * tch, edge_o = bsh_o + 4u * tch;
-    // exact-path queues [pair mod 3][consumer warp]: counts, then EXM_SLOWQ int2 entries (storage index of the
-    // tap; template | boundary flag << 30 | random-draw flag << 29)
-    const unsigned qcnt_o = edge_o + 4u * (2 * 2 * 8 * 32), qent_o = qcnt_o + 4u * 3 * 32;
-    int *qcnt = (int *)(smem + qcnt_o);
-    const int2 *qent = (const int2 *)(smem + qent_o);
-    auto edge_off = [&](int par, int b2) { return edge_o + 4u * (unsigned)((par * 2 + b2) * 8 * NC); };
-    __shared__ int bl_sh[2];
-    __shared__ unsigned bad_sh;
-
-    // block -> (lag, node, template chunk), lags outermost so the blocks of one lag run together
-    const int c_idx = blockIdx.x % a.nch;
-    const int k = (blockIdx.x / a.nch) % a.nn;
-    const int rl = blockIdx.x / (a.nch * a.nn), r = a.r0 + rl;
-    const int lo0 = max(a.mlo[k], a.m_base), hi0 = min(a.mhi[k], a.m_base + a.nmc);
+    // block -> (lag, template chunk, node, part of the plane pairs): the blocks of one (lag, chunk), which
+    // read the same descriptors, run together; after a lag's regular blocks those of its boundary points
+    int blk = blockIdx.x;
+    const int part_i = blk % a.nparts;
+    blk /= a.nparts;
+    const int per_r = a.nn * a.nch + a.nbn * a.nchb;
+    const int rl = blk / per_r, r = a.r0 + rl;
+    blk %= per_r;
+    const bool bnd = blk >= a.nn * a.nch;
+    if (bnd) blk -= a.nn * a.nch;
+    const int bi = bnd ? blk % a.nbn : 0;
+    const int k = bnd ? a.bn_k[bi] : blk % a.nn;
+    const int tch = bnd ? a.tchb : a.tch;
+    const int c_idx = bnd ? blk / a.nbn : blk / a.nn;
+    const int lo0 = bnd ? a.bn_lo[bi] : max(a.mlo[k], a.m_base);
+    const int hi0 = bnd ? a.bn_hi[bi] : min(a.mhi[k], a.m_base + a.nmc);
     const int lo = lo0 + c_idx * tch;
     const int hi = min(hi0, lo + tch);
     if (lo >= hi) return;
     const int n = hi - lo;
+    const int p_beg = part_i * EXM_NPAIR / a.nparts, np = (part_i + 1) * EXM_NPAIR / a.nparts - p_beg;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned acc_o = 3 * SLOT_B + 64;
+    float *acc = gsm_f(acc_o);
+    const unsigned bcf_o = acc_o + 4u * EXM_ACC_F * tch, bsh_o = bcf_o + 4u * tch;   // boundary blocks
+    const unsigned edge_o = acc_o + 4u * EXM_ACC_F * a.tch;
+    const unsigned qcnt_o = edge_o + EXM_EDGE_B, qent_o = qcnt_o + EXM_QCNT_B;
+    int *qcnt = (int *)(smem + qcnt_o);
+    const int2 *qent = (const int2 *)(smem + qent_o);
+    auto edge_off = [&](int par) { return edge_o + 4u * (unsigned)(par * EXM_EDGE_F * NC); };
+    __shared__ unsigned bad_sh;
 
-    if (tid == 0) {
-        bl_sh[0] = n;
-        bl_sh[1] = 0;
-        bad_sh = 0;
-    }
-    __syncthreads();
+    if (tid == 0) bad_sh = 0;
     // the node's window: column C0, first row R0 = Rh + cki clamped to the table; a tap's window row
-    // is its beta-hat row from Rh (in the descriptor), plus the carry of the node's beta fraction, plus sh
+    // is its beta-hat row from Rh (in the descriptor), plus the carry of the beta fractions, plus sh
     const int C0 = a.win[0], R0 = a.win[1 + k], Rh = a.win[1 + EXM_MAX_NODES];
     const int sh = Rh + a.cki[k] - R0;
     for (int j = tid; j < n; j += NW * 32) {
 #pragma unroll
-        for (int q = 0; q < 6; ++q) {
-            acc[(3 * q) * tch + j] = -1e30f;
-            acc[(3 * q + 1) * tch + j] = 0.f;
-            acc[(3 * q + 2) * tch + j] = 0.f;
+        for (int q = 0; q < 3; ++q) {
+            acc[(2 * q) * tch + j] = EXM_MNONE;
+            acc[(2 * q + 1) * tch + j] = 0.f;
         }
-        bsh[j] = EXM_BSH_NONE;
-        if (a.bnode[lo + j] == k) {
-            const double cbv = a.cb[lo + j];
-            const double f = floor(cbv);
-            bsh[j] = (int)f - a.cki[k] + sh;
-            bcf[j] = (float)(cbv - f);
-            atomicMin(&bl_sh[0], j);
-            atomicMax(&bl_sh[1], j + 1);
+        if (bnd) {
+            int bs = EXM_BSH_NONE;
+            unsigned bf = 0u;
+            if (a.bnode[lo + j] == k) {
+                const double cbv = a.cb[lo + j];
+                const double f = floor(cbv);
+                const int rows = (int)f - a.cki[k] + sh;
+                bs = EXM_BSH_FAR;   // no tap reaches the window: every one takes the exact path
+                if (abs(rows) <= EXM_MAX_SHIFT) {
+                    bs = rows * TabElem<TE>::wd;
+                    bf = __double2uint_rn((cbv - f) * 8388608.0);
+                }
+            }
+            ((int *)gsm_f(bsh_o))[j] = bs;
+            ((unsigned *)gsm_f(bcf_o))[j] = bf;
         }
     }
     if (tid == 0) {
@@ -559,34 +643,33 @@ __global__ void __launch_bounds__(NW * 32, 1) k_gather_planes(const __grid_const
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    const int blo = bl_sh[0], bhi = bl_sh[1];
     unsigned n_slow = 0, n_bnd = 0;
 
     if (warp == NC) {
         // ---------------------------------------------------------------- producer
         const int32_t *tsr_all = a.tside + (long long)rl * a.per_lag;
+        const int nplanes = np + 1;
         int issued = 0;
         if (a.stage) {
             if (lane == 0)
-                for (int q = 0; q < 3 && q < a.nphif; ++q)
-                    tma_load_plane(&tmap, &full[q], win + q * SLOT, C0, R0, q, r, k, SLOT_B);
-            issued = min(3, a.nphif);
+                for (int q = 0; q < 3 && q < nplanes; ++q)
+                    tma_load_plane(&tmap, &full[q], win + q * SLOT, C0, R0, p_beg + q, r, k, SLOT_B);
+            issued = min(3, nplanes);
         }
         bool ok = true;
-        for (int p = 0; p < EXM_NPAIR; ++p) {
+        for (int p = 0; p < np; ++p) {
             ok = ok && __all_sync(0xffffffffu, mbar_wait(&done[p & 1], (p >> 1) & 1, a.err, a.wait_cycles));
             if (!ok) break;
-            fold_edges(gsm_f(edge_off(p & 1, 0)), NC, acc + 6 * tch, acc + 7 * tch, acc + 8 * tch, n);
-            if (blo < bhi)
-                fold_edges(gsm_f(edge_off(p & 1, 1)), NC, acc + 15 * tch, acc + 16 * tch, acc + 17 * tch, n);
+            fold_edges(gsm_f(edge_off(p & 1)), NC, acc + 4 * tch, acc + 5 * tch, n);
             __syncwarp();
             // plane p is no longer needed anywhere: its slot takes plane p + 3
-            if (a.stage && p + 3 < a.nphif) {
-                if (lane == 0) tma_load_plane(&tmap, &full[p % 3], win + (p % 3) * SLOT, C0, R0, p + 3, r, k, SLOT_B);
+            if (a.stage && p + 3 < nplanes) {
+                if (lane == 0)
+                    tma_load_plane(&tmap, &full[p % 3], win + (p % 3) * SLOT, C0, R0, p_beg + p + 3, r, k, SLOT_B);
                 ++issued;
             }
             // the exact-path taps the consumers queued for pair p: 32 lanes compute them, lane 0 merges them
-            // in warp and queue order into the producer's sets (the consumers reuse these queues at pair
+            // in warp and queue order into the producer's set (the consumers reuse these queues at pair
             // p + 3, after plane p + 4, which is staged only after this)
             {
                 const int par = p % 3;
@@ -602,7 +685,7 @@ __global__ void __launch_bounds__(NW * 32, 1) k_gather_planes(const __grid_const
                 for (int b0 = 0; b0 < total; b0 += 32) {
                     const int i = b0 + lane;
                     double v = 0.0;
-                    int tr = 0, bnd = 0;
+                    int tr = 0;
                     int wi = 0;   // the warp whose entries [excl, incl) hold i (shuffles kept converged)
                     for (int l = 1; l < NC; ++l) {
                         const int el = __shfl_sync(0xffffffffu, excl, l);
@@ -612,7 +695,6 @@ __global__ void __launch_bounds__(NW * 32, 1) k_gather_planes(const __grid_const
                     if (i < total) {
                         const int2 e = qent[(par * 32 + wi) * EXM_SLOWQ + (i - wexcl)];
                         const int il = e.y & 0x1FFF;
-                        bnd = (e.y >> 30) & 1;
                         const int tm = tsr_all[e.x];
                         v = bnd ? slow_tap<true, TE>(a, il, tm, k, r, a.m_base, a.tsc[k])
                                 : slow_tap<false, TE>(a, il, tm, k, r, a.m_base, a.tsc[k]);
@@ -622,16 +704,15 @@ __global__ void __launch_bounds__(NW * 32, 1) k_gather_planes(const __grid_const
                     const int nb2 = min(32, total - b0);
                     for (int qq = 0; qq < nb2; ++qq) {
                         const double vq = __shfl_sync(0xffffffffu, v, qq);
-                        const int tq = __shfl_sync(0xffffffffu, tr, qq), bq = __shfl_sync(0xffffffffu, bnd, qq);
+                        const int tq = __shfl_sync(0xffffffffu, tr, qq);
                         if (lane == 0 && tq >= 0 && tq < n) {
-                            float B, E;
-                            split_double(vq, B, E);
-                            float *F = acc + (bq ? 15 : 6) * tch;
-                            float b = F[tq], x = F[tch + tq], sv = F[2 * tch + tq];
-                            lse_merge(b, x, sv, B, E, 1.f);
-                            F[tq] = b;
-                            F[tch + tq] = x;
-                            F[2 * tch + tq] = sv;
+                            float m2, S2;
+                            split_double(vq, m2, S2);
+                            float *F = acc + 4 * tch;
+                            float m = F[tq], S = F[tch + tq];
+                            ms_merge(m, S, m2, S2);
+                            F[tq] = m;
+                            F[tch + tq] = S;
                         }
                     }
                 }
@@ -655,20 +736,33 @@ __global__ void __launch_bounds__(NW * 32, 1) k_gather_planes(const __grid_const
         rc.bsh = bsh_o;
         rc.bcf = bcf_o;
         rc.accst = 4u * tch;
+        rc.ng = a.ng;
         rc.lo = lo;
         rc.m_base = a.m_base;
         rc.n = n;
-        rc.sh = sh;
-        rc.up = min(EXM_WB - 2, a.nb - 2 - R0);
-        rc.edge = a.nb - 2 - R0;
+        // rows 0 .. up of the window are served: up + 1 must be in the window, and the table's last row
+        // pair, where the reference clamps beta just below the top, is left to the exact path
+        const int up = min(a.wb - 2, a.nb - 3 - R0);
+        const bool near = bnd || abs(sh) <= EXM_MAX_SHIFT;
+        rc.sh = near ? sh * TabElem<TE>::wd : EXM_BSH_FAR;
+        rc.lim = (up >= 0 && near) ? (unsigned)((up + 1) * TabElem<TE>::wd) : 0u;
         rc.ckf = a.ckf[k];
         rc.sc = a.tsc[k];
         rc.k = k;
         rc.r = r;
         rc.lw = a.lw;
-        const int base_i = lo - a.m_base;   // chunk-local index of template lo
+        rc.wr = a.wr;
+        // the run offsets are loaded two pairs ahead, a warp's first descriptors and end templates one
+        const int *offp = offr + (long long)p_beg * (a.nmc + 1) + (lo - a.m_base);
+        open_share<NC>(rc, offp[0], offp[n], 0);
+        int nb0 = 0, nb1 = 0;
+        if (np > 1) {
+            offp += a.nmc + 1;
+            nb0 = offp[0];
+            nb1 = offp[n];
+        }
         bool ok = true;
-        for (int p = 0; p < EXM_NPAIR; ++p) {
+        for (int p = 0; p < np; ++p) {
             // warp-uniform: the lanes go on to shuffles together
             ok = ok && __all_sync(0xffffffffu, mbar_wait(&full[p % 3], (p / 3) & 1, a.err, a.wait_cycles));
             ok = ok && __all_sync(0xffffffffu,
@@ -677,29 +771,49 @@ __global__ void __launch_bounds__(NW * 32, 1) k_gather_planes(const __grid_const
             __syncwarp();
             rc.qn = qcnt_o + 4u * ((p % 3) * 32 + warp);
             rc.q = qent_o + 8u * (((p % 3) * 32 + warp) * EXM_SLOWQ);
-            if (ok) {
+            if (!ok) {   // no work: empty edge slots for the producer
+                rc.tF = rc.tL = -1;
+                rc.beg = rc.end = 0;
+            }
+            open_edge(rc, edge_off(p & 1) + 4u * EXM_EDGE_F * warp);
+            if (rc.beg < rc.end) {
                 rc.s0 = (p % 3) * SLOT_B;
                 rc.s1 = ((p + 1) % 3) * SLOT_B;
-                const int *offp = offr + p * (a.nmc + 1) + base_i;
-                rc.acc = acc_o + 4u * (3u * (p & 1) * tch);
-                warp_share<false, GRP, NC, TE>(a, rc, offp[0], offp[n], edge_off(p & 1, 0), p, n_slow);
-                if (blo < bhi) {
-                    rc.acc = acc_o + 4u * ((9u + 3u * (p & 1)) * tch);
-                    const int bb = offp[blo], be = offp[bhi];
-                    n_bnd += (lane == 0 && warp == 0) ? (unsigned)(be - bb) : 0u;
-                    warp_share<true, GRP, NC, TE>(a, rc, bb, be, edge_off(p & 1, 1), p, n_slow);
-                }
-            } else if (lane == 0) {   // no work: empty edge slots for the producer
-                for (int b2 = 0; b2 < 2; ++b2) {
-                    float *e = gsm_f(edge_off(p & 1, b2)) + 8 * warp;
-                    e[3] = __int_as_float(-1);
-                    e[7] = __int_as_float(-1);
-                }
+                rc.acc = acc_o + 4u * (2u * (p & 1) * tch);
+                if (bnd)
+                    process_run<true, PF, TE>(a, rc, n_slow);
+                else
+                    process_run<false, PF, TE>(a, rc, n_slow);
             }
             __syncwarp();
             mbar_arrive(&done[p & 1]);
+            if (p + 1 < np) {
+                const int b0 = nb0, b1 = nb1;
+                if (p + 2 < np) {
+                    offp += a.nmc + 1;
+                    nb0 = offp[0];
+                    nb1 = offp[n];
+                }
+                open_share<NC>(rc, b0, b1, p + 1);
+            }
         }
         if (!ok && lane == 0) atomicOr(&bad_sh, 1u);
+    }
+    __syncthreads();
+    const bool ok = bad_sh == 0;
+    const long long prow = a.ntau * a.nparts;   // partial sums per node and template
+    for (int j = tid; j < n; j += NW * 32) {
+        // the three sets of a template: both pair parities, and the producer's
+        float m = acc[j], S = acc[tch + j];
+        ms_merge(m, S, acc[2 * tch + j], acc[3 * tch + j]);
+        ms_merge(m, S, acc[4 * tch + j], acc[5 * tch + j]);
+        const double v = (ok && S > 0.f) ? (double)m + log((double)S) : -INFINITY;
+        if (!bnd) {
+            a.part[(k * prow + r * a.nparts + part_i) * a.nm_total + lo + j] = v;
+        } else if (a.bnode[lo + j] == k) {
+            a.part[(a.nn * prow + r * a.nparts + part_i) * a.nm_total + lo + j] = v;
+            if (part_i == 0) n_bnd += (unsigned)a.nwalk;
+        }
     }
     if (a.stats) {
         const unsigned sl_ = __reduce_add_sync(0xffffffffu, n_slow), bd_ = __reduce_add_sync(0xffffffffu, n_bnd);
@@ -708,50 +822,34 @@ __global__ void __launch_bounds__(NW * 32, 1) k_gather_planes(const __grid_const
             atomicAdd(&a.stats[1], (unsigned long long)bd_);
         }
     }
-    __syncthreads();
-    const bool ok = bad_sh == 0;
-    for (int j = tid; j < n; j += NW * 32) {
-        // the three sets of a template: both pair parities and the folded edges
-        float B = acc[j], E = acc[tch + j], S = acc[2 * tch + j];
-        lse_merge(B, E, S, acc[3 * tch + j], acc[4 * tch + j], acc[5 * tch + j]);
-        lse_merge(B, E, S, acc[6 * tch + j], acc[7 * tch + j], acc[8 * tch + j]);
-        const double v = (ok && S > 0.f) ? (double)B + (double)E + log((double)S) : -INFINITY;
-        a.part[((long long)k * a.ntau + r) * a.nm_total + lo + j] = v;
-        if (j >= blo && j < bhi && a.bnode[lo + j] == k) {
-            float B2 = acc[9 * tch + j], E2 = acc[10 * tch + j], S2 = acc[11 * tch + j];
-            lse_merge(B2, E2, S2, acc[12 * tch + j], acc[13 * tch + j], acc[14 * tch + j]);
-            lse_merge(B2, E2, S2, acc[15 * tch + j], acc[16 * tch + j], acc[17 * tch + j]);
-            const double v2 = (ok && S2 > 0.f) ? (double)B2 + (double)E2 + log((double)S2) : -INFINITY;
-            a.part[((long long)a.nn * a.ntau + r) * a.nm_total + lo + j] = v2;
-        }
-    }
 }
 
-// launch shapes the autotuner chooses from: (warps per block, taps per register group)
+// ------------------------------------------------------------------ launch
+
+// launch shapes the autotuner chooses from: warps per block including the producer, and the pairs of taps
+// whose window reads a lane has in flight; the first is the default of an untuned context
 struct GatherCfg {
-    int nw, grp;
+    int nw, pf;
 };
-// warps incl. producer x taps per register group; the first is the default of an untuned context
-static const GatherCfg kGatherCfgs[] = {{28, 1}, {16, 2}, {24, 2}, {24, 1}, {20, 2}};
+static const GatherCfg kGatherCfgs[] = {{20, 2}, {28, 1}, {16, 2}, {24, 2}, {24, 1}};
 static const int kNumGatherCfgs = (int)(sizeof(kGatherCfgs) / sizeof(kGatherCfgs[0]));
 
-template <int NW, int GRP0, typename TE>
+template <int NW, int PF, typename TE>
 static void launch_planes(exm_ctx *ctx, const PlaneArgs &a, dim3 grid, size_t smem)
 {
-    constexpr int GRP = GRP0 < TPL ? GRP0 : TPL;   // a register group never exceeds a lane's taps
-    exm_allow_smem(ctx, (const void *)k_gather_planes<NW, GRP, TE>, smem);
-    k_gather_planes<NW, GRP, TE><<<grid, NW * 32, smem, ctx->stream>>>(ctx->tmap, a);
+    exm_allow_smem(ctx, (const void *)k_gather_planes<NW, PF, TE>, smem);
+    k_gather_planes<NW, PF, TE><<<grid, NW * 32, smem, ctx->stream>>>(ctx->tmap, a);
 }
 
 template <typename TE>
 static void launch_cfg_t(exm_ctx *ctx, int cfg, const PlaneArgs &a, dim3 grid, size_t smem)
 {
     switch (cfg) {
-    case 0: launch_planes<28, 1, TE>(ctx, a, grid, smem); break;
-    case 1: launch_planes<16, 2, TE>(ctx, a, grid, smem); break;
-    case 2: launch_planes<24, 2, TE>(ctx, a, grid, smem); break;
-    case 3: launch_planes<24, 1, TE>(ctx, a, grid, smem); break;
-    default: launch_planes<20, 2, TE>(ctx, a, grid, smem); break;
+    case 0: launch_planes<20, 2, TE>(ctx, a, grid, smem); break;
+    case 1: launch_planes<28, 1, TE>(ctx, a, grid, smem); break;
+    case 2: launch_planes<16, 2, TE>(ctx, a, grid, smem); break;
+    case 3: launch_planes<24, 2, TE>(ctx, a, grid, smem); break;
+    default: launch_planes<24, 1, TE>(ctx, a, grid, smem); break;
     }
 }
 
@@ -767,25 +865,72 @@ static void launch_cfg(exm_ctx *ctx, int cfg, const PlaneArgs &a, dim3 grid, siz
 
 int exm_gather_num_cfgs() { return kNumGatherCfgs; }
 
-static size_t planes_smem(int tch, int dtype)
+static size_t planes_smem(int tch, int wb, int dtype)
 {
-    const size_t slot = (size_t)EXM_WB * exm_dtype_wd(dtype) * exm_dtype_bytes(dtype);
-    // 6 accumulator sets of 3 floats, bcf, bsh; edge slots; exact-path queue counts and entries
-    return 3 * slot + 64 + (size_t)tch * 20 * 4 + 2 * 2 * 8 * 32 * 4 + 3 * 32 * 4 + 3 * 32 * EXM_SLOWQ * 8;
+    return 3 * (size_t)wb * exm_dtype_wd(dtype) * exm_dtype_bytes(dtype) + EXM_GATHER_FIXED_B + (size_t)tch * EXM_ACC_F * 4;
 }
 
-// the most templates a block can hold in shared memory next to the staged planes
-static int planes_tch_max(exm_ctx *ctx)
+// templates a gather block may hold next to windows of wb rows (2 KB are left for the static shared memory)
+static int planes_tch_max(const exm_ctx *ctx, int wb)
 {
-    const size_t slot = (size_t)EXM_WB * exm_dtype_wd(ctx->dtype) * exm_dtype_bytes(ctx->dtype);
-    const size_t fixed = 3 * slot + 64 + 2 * 2 * 8 * 32 * 4 + 3 * 32 * 4 + 3 * 32 * EXM_SLOWQ * 8 + 2048;   // + static
+    const size_t fixed = planes_smem(0, wb, ctx->dtype) + 2048;
     const size_t room = ctx->smem_optin > fixed ? ctx->smem_optin - fixed : 0;
-    return (int)std::min<size_t>(EXM_TCH, room / (20 * 4) / 16 * 16);
+    return (int)std::min<size_t>(EXM_TCH, room / (EXM_ACC_F * 4) / 16 * 16);
+}
+
+// templates per gather block: pct / 150 of the most that still gives every SM eight blocks (a block's start,
+// the waits at each plane pair and the staging of its windows are paid once for all its templates), between
+// 256 and EXM_TCH_PLAN at 150
+static int planes_tch(const exm_ctx *ctx, const ChunkInfo &ci, int rc, int pct, int *maxn_out)
+{
+    long long pairs = 0;
+    int maxn = 0;
+    for (int k = 0; k < ctx->nn; ++k) {
+        const int lo = std::max(ctx->mlo[k], ci.m_base), hi = std::min(ctx->mhi[k], ci.m_base + ci.nmc);
+        pairs += std::max(0, hi - lo);
+        maxn = std::max(maxn, hi - lo);
+    }
+    *maxn_out = maxn;
+    long long tch = pairs * rc / std::max(1, 8 * ctx->sm_count);
+    tch = std::min<long long>(std::max<long long>(tch, 256), EXM_TCH_PLAN);
+    tch = std::min<long long>(tch * pct / 150, EXM_TCH);
+    tch = std::max<long long>(1, std::min<long long>(tch, maxn));
+    return (int)((tch + 15) / 16 * 16);
+}
+
+// The windows' height and the descriptors' chunk, which the tap build and the gather share.  Rows: the most that
+// fit beside the accumulators of the templates a default block takes (at least EXM_WB_MIN, at most
+// EXM_WB_MAX): every row more leaves fewer taps to the exact path.  Groups per lane: 4 (chunks of 512 taps),
+// fewer when a plane pair of a block has too few taps to give every warp a chunk.
+void exm_gather_plan(const exm_ctx *ctx, const ChunkInfo &ci, int rc, int *wb_out, int *ng_out)
+{
+    int maxn = 0;
+    const int tch = planes_tch(ctx, ci, rc, 150, &maxn);
+    const size_t fixed = EXM_GATHER_FIXED_B + 2048 + (size_t)tch * EXM_ACC_F * 4;
+    const size_t row = 3 * (size_t)exm_dtype_wd(ctx->dtype) * exm_dtype_bytes(ctx->dtype);
+    int wb = (int)((ctx->smem_optin - fixed) / row) / 8 * 8;
+    wb = std::min(wb, std::max(EXM_WB_MIN, (ctx->nb + 7) / 8 * 8));
+    *wb_out = std::max(EXM_WB_MIN, std::min(wb, EXM_WB_MAX));
+    const double taps = (double)std::min(tch, std::max(maxn, 1)) * ci.nwalk / EXM_NPAIR;   // of a pair of a block
+    *ng_out = taps >= 12288 ? 4 : (taps >= 3584 ? 2 : 1);
+}
+
+// Parts of the 48 plane pairs a (node, lag, template chunk) is split into, each a block of its own: one, or
+// more when the launch has too few blocks to keep the SMs busy to the end.
+int exm_gather_parts(const exm_ctx *ctx, int nmc, int m_base, int nwalk, int rc)
+{
+    (void)nwalk;
+    int maxn = 0;
+    ChunkInfo ci{m_base, nmc, nwalk, 0, 0.f};
+    const int tch = planes_tch(ctx, ci, rc, 150, &maxn);
+    const long long blocks = (long long)rc * ctx->nn * ((maxn + tch - 1) / std::max(tch, 1));
+    const long long waves = blocks / std::max(1, ctx->sm_count);
+    return waves >= 8 ? 1 : (waves >= 4 ? 2 : 4);
 }
 
 void exm_run_gather_planes(exm_ctx *ctx, exm_slot &sl, const ChunkInfo &ci, int r0, int rc)
 {
-    if (!ctx->tmap_ok) EXM_THROW(EXM_ERR_STATE, "tensor map of the store is not set");
+    exm_make_tmap(ctx, sl.wb);
     PlaneArgs a;
     memset(&a, 0, sizeof(a));
     a.desc = (const uint4 *)sl.desc.p;
@@ -808,7 +953,7 @@ void exm_run_gather_planes(exm_ctx *ctx, exm_slot &sl, const ChunkInfo &ci, int 
     a.err = (unsigned *)sl.dev_err.p;
     a.stats = (unsigned long long *)ctx->d_stats.p;
     a.tstride = (long long)ctx->tstride;
-    a.per_lag = exm_desc_pitch((long long)ci.nmc * ci.nwalk);   // storage stride of a lag's descriptors
+    a.per_lag = exm_desc_pitch(ci.nmc, ci.nwalk);   // storage stride of a lag's descriptors
     a.nn = ctx->nn;
     a.ntau = ctx->ntau;
     a.nphif = ctx->nphif;
@@ -817,10 +962,15 @@ void exm_run_gather_planes(exm_ctx *ctx, exm_slot &sl, const ChunkInfo &ci, int 
     a.ndp = ctx->ndp;
     a.nt = ctx->nt;
     a.nmc = ci.nmc;
+    a.nwalk = ci.nwalk;
     a.m_base = ci.m_base;
     a.nm_total = ctx->nm;
     a.r0 = r0;
+    a.wb = sl.wb;
+    a.ng = sl.ng;
+    a.nparts = sl.nparts;
     a.lw = ci.lw;
+    a.wr = (float)std::exp((double)ci.lw);
     a.rph = EXM_NPHI / 6.283185307179586;
     a.rdb = 2.0 / ctx->dbeta;
     a.rdd = 1.0 / ctx->ddelta;
@@ -830,27 +980,35 @@ void exm_run_gather_planes(exm_ctx *ctx, exm_slot &sl, const ChunkInfo &ci, int 
     for (int k = 0; k < ctx->nn; ++k) {
         const double f = std::floor(ctx->ck[k]);
         a.cki[k] = (int)f;
-        a.ckf[k] = (float)(ctx->ck[k] - f);
+        a.ckf[k] = (unsigned)std::nearbyint((ctx->ck[k] - f) * 8388608.0);
         a.tsc[k] = ctx->tscale[k];
     }
-    // templates per block: about one wave of blocks per lag, so that the descriptors of the lag
-    // in flight stay in L2; at most EXM_TCH (shared-memory accumulators)
-    long long pairs = 0;
     int maxn = 0;
-    for (int k = 0; k < ctx->nn; ++k) {
-        const int lo = std::max(ctx->mlo[k], ci.m_base), hi = std::min(ctx->mhi[k], ci.m_base + ci.nmc);
-        pairs += std::max(0, hi - lo);
-        maxn = std::max(maxn, hi - lo);
-    }
+    int tch = planes_tch(ctx, ci, rc, ctx->gather_chunk_pct, &maxn);
     if (maxn <= 0) return;
-    int tch = (int)((pairs + ctx->sm_count - 1) / ctx->sm_count);
-    tch = (int)((long long)tch * ctx->gather_chunk_pct / 100);
-    tch = std::max(tch, 256);
-    tch = std::min(((tch + 15) / 16) * 16, planes_tch_max(ctx));
-    a.tch = tch;
+    tch = std::min(tch, planes_tch_max(ctx, sl.wb));
     a.nch = (maxn + tch - 1) / tch;
-    const size_t smem = planes_smem(tch, ctx->dtype);
-    dim3 grid(rc * ctx->nn * a.nch);
+    tch = std::min(tch, ((maxn + a.nch - 1) / a.nch + 15) / 16 * 16);   // equal chunks
+    a.tch = tch;
+    // boundary points: the templates of each node that has some, in chunks whose extra arrays fit the same space
+    int maxb = 0;
+    for (int k = 0; k < ctx->nn; ++k) {
+        int lo = -1, hi = -1;
+        for (int i = ci.m_base; i < ci.m_base + ci.nmc; ++i)
+            if (ctx->bnode[i] == k) {
+                if (lo < 0) lo = i;
+                hi = i + 1;
+            }
+        if (lo < 0) continue;
+        a.bn_k[a.nbn] = k;
+        a.bn_lo[a.nbn] = lo;
+        a.bn_hi[a.nbn++] = hi;
+        maxb = std::max(maxb, hi - lo);
+    }
+    a.tchb = std::max(1, tch * EXM_ACC_F / EXM_ACCB_F);
+    a.nchb = (maxb + a.tchb - 1) / a.tchb;
+    const size_t smem = planes_smem(tch, sl.wb, ctx->dtype);
+    dim3 grid(rc * (ctx->nn * a.nch + a.nbn * a.nchb) * a.nparts);
     const int cfg = (ctx->gather_cfg >= 0 && ctx->gather_cfg < kNumGatherCfgs) ? ctx->gather_cfg : 0;
     launch_cfg(ctx, cfg, a, grid, smem);
     EXM_CUDA(cudaGetLastError());

@@ -8,10 +8,13 @@
 
 #include "common.cuh"
 
-// staging window of one (node, lag, phase plane): rows of beta x columns of Delta
-#define EXM_WB 80
-#define EXM_WD 164     // float32 tables: row pitch = 4 banks mod 32, neighbouring rows start on different banks
-#define EXM_WD16 168   // 16-bit tables: a multiple of 8 elements (16-byte TMA rows), pitch 20 banks mod 32
+// staging window of one (node, lag, phase plane): rows of beta x columns of Delta.  The row pitch is a
+// multiple of the 32 banks, so the bank of a value depends on its column alone.  The rows are chosen per launch
+// (exm_gather_plan).
+#define EXM_WD 160     // float32 tables
+#define EXM_WD16 192   // 16-bit tables
+#define EXM_WB_MIN 80
+#define EXM_WB_MAX 160
 
 // Table elements as stored: float32, or 16-bit with a per-node scale (value = scale * element;
 // the scale is a power of two for float16 and 1 for bfloat16, so the product is exact).
@@ -43,27 +46,43 @@ inline size_t exm_dtype_bytes(int dtype) { return dtype == EXM_DTYPE_F32 ? 4 : 2
 inline int exm_dtype_wd(int dtype) { return dtype == EXM_DTYPE_F32 ? EXM_WD : EXM_WD16; }
 inline int exm_dtype_calign(int dtype) { return dtype == EXM_DTYPE_F32 ? 4 : 8; }
 #define EXM_TCH 2048        // templates per gather block
+#define EXM_TCH_PLAN 1024   // ... by default
 
-// Tap descriptors of one lag, sorted by (plane pair, template), are stored in chunks of
-// EXM_DCH = 32 * EXM_TPL.  The gather's lane l takes the consecutive taps l*TPL .. l*TPL+TPL-1
-// of a chunk (so equal templates meet in registers), and they are stored lane-interleaved --
-// tap i of lane l at i*32 + l -- so that every load instruction of a warp reads 32 consecutive
-// descriptors (512 bytes) instead of 32 scattered cache lines.
-#ifndef EXM_TPL
-#define EXM_TPL 16
-#endif
-#define EXM_DCH (32 * EXM_TPL)
-static_assert((EXM_TPL & (EXM_TPL - 1)) == 0, "taps per lane must be a power of two");
+// Tap descriptors of one lag are sorted by (plane pair, template) and each (pair, template) run is padded to
+// whole groups of EXM_GT taps, so that every group has one template.  They are stored in chunks of 32 EXM_GT ng
+// taps (ng groups per lane: 1, 2 or 4, exm_gather_plan).  The gather's lane l takes the consecutive groups
+// l ng .. l ng + ng - 1 of a chunk (so equal templates meet in registers), and they are stored
+// lane-interleaved -- the i-th tap of lane l at i 32 + l -- so that every load instruction of a warp reads 32
+// consecutive descriptors (512 bytes) instead of 32 scattered cache lines.
+#define EXM_GT 4
+#define EXM_NG_MAX 4
+#define EXM_CH_MAX (32 * EXM_GT * EXM_NG_MAX)
+
+// A descriptor's fourth word: window offset o0 = (beta-hat row - Rh) * columns + (Delta column - C0) in the upper
+// 19 bits (signed), template in the lower 13.  Two offsets mark special taps: EXM_O_FAR a tap outside every window (the
+// exact path), EXM_O_PAD a padding entry.  Real offsets lie within +-1024 rows, and a node's shift of more
+// than EXM_MAX_SHIFT rows leaves all its taps to the exact path, so neither mark can reach a window.
+#define EXM_O_FAR 262143
+#define EXM_O_PAD (-262144)
+#define EXM_DESC_PAD 0x80000000u                    // fourth word of a padding entry (template 0)
+#define EXM_DESC_REAL ((int)((unsigned)(-200000) << 13))   // words at or above (signed) are real taps
+#define EXM_MAX_SHIFT 1100
+#define EXM_BSH_FAR (1 << 28)                       // shift of a node no tap of which reaches the window
 
 // storage index of the descriptor at sorted position j (within its lag)
-__host__ __device__ __forceinline__ long long exm_desc_phys(long long j)
+__host__ __device__ __forceinline__ long long exm_desc_phys(long long j, int ng)
 {
-    const long long q = j & (EXM_DCH - 1);
-    return (j - q) + (q % EXM_TPL) * 32 + q / EXM_TPL;
+    const int tpl = EXM_GT * ng;
+    const long long q = j & (32 * tpl - 1);
+    return (j - q) + (q & (tpl - 1)) * 32 + q / tpl;
 }
 
-// descriptors per lag as stored: whole chunks
-inline long long exm_desc_pitch(long long per_lag) { return (per_lag + EXM_DCH - 1) / EXM_DCH * EXM_DCH; }
+// descriptors per lag as stored: every run padded to whole groups, whole chunks
+inline long long exm_desc_pitch(long long nmc, long long nwalk)
+{
+    const long long runs = nmc * std::min<long long>(EXM_NPAIR, nwalk);
+    return (nmc * nwalk + runs * (EXM_GT - 1) + EXM_CH_MAX - 1) / EXM_CH_MAX * EXM_CH_MAX;
+}
 #define EXM_MAX_CHUNK 8192  // templates per pass (13-bit template field of a descriptor)
 #define EXM_MAX_NODES 64
 #define EXM_HB_LO (-1024)   // beta-hat histogram covers [-1024, 1024)
@@ -79,15 +98,14 @@ struct TapGeom {
 
 // The per-tap quantities that do not depend on the node (the reference computes
 // them per node, exmarg/search/gather.py:50-82): the plane pair p and the weight w
-// of plane p + 1, beta-hat = ln|z_L| 2/dbeta - ln(u)/dbeta as floor + fraction,
-// and the Delta coordinate of the unclamped-beta case as (d0, fd).
+// of plane p + 1, beta-hat = ln|z_L| 2/dbeta - ln(u)/dbeta as floor + fraction (23-bit fixed point,
+// rounded: 2^23 carries into the row when a node's fraction is added), and the Delta coordinate of the unclamped-beta case as (d0, fd).
 // ln|z| enters as its float32 value plus the filter's float32 residual (llo, hlo: ln|z| - float(ln|z|), zero for
 // trajectories given as float32), so beta-hat and Delta see the filter's float64 value; the phases stay float32
 // and are subtracted in float32, as the reference does.
-__device__ __forceinline__ void exm_tap_geom(float2 l, float2 h, float llo, float hlo, double boff, const TapGeom &g,
-                                             int &p, float &w, int &ib, float &fb, int &d0, float &fd)
+__device__ __forceinline__ void exm_tap_phase(float phL, float phH, const TapGeom &g, int &p, float &w)
 {
-    double x3 = (double)(h.y - l.y) * g.rph;   // float32 difference, float64 scale, as the reference
+    double x3 = (double)(phH - phL) * g.rph;   // float32 difference, float64 scale, as the reference
     if (x3 < 0.0) x3 += EXM_NPHI;
     if (x3 >= EXM_NPHI) x3 -= EXM_NPHI;
     int c0 = (int)x3;
@@ -101,11 +119,28 @@ __device__ __forceinline__ void exm_tap_geom(float2 l, float2 h, float llo, floa
         p = EXM_NPHI - 1 - c0;
         w = (float)(1.0 - fc);
     }
-    const double aL = (double)l.x + (double)llo, aH = (double)h.x + (double)hlo;
-    const double bh = aL * g.rdb + boff;
+}
+
+__device__ __forceinline__ void exm_tap_beta(float lqL, float lqLlo, double boff, const TapGeom &g, int &ib, unsigned &fb)
+{
+    const double bh = ((double)lqL + (double)lqLlo) * g.rdb + boff;
     const double fl = floor(bh);
     ib = (int)fmax(fmin(fl, 1023.0), -1024.0);
-    fb = (float)(bh - fl);
+    fb = __double2uint_rn((bh - fl) * 8388608.0);
+}
+
+__device__ __forceinline__ int exm_tap_row(float lqL, float lqLlo, double boff, const TapGeom &g)
+{
+    int ib;
+    unsigned fb;
+    exm_tap_beta(lqL, lqLlo, boff, g, ib, fb);
+    return ib;
+}
+
+__device__ __forceinline__ void exm_tap_delta(float lqL, float lqLlo, float lqH, float lqHlo, const TapGeom &g, int &d0,
+                                              float &fd)
+{
+    const double aL = (double)lqL + (double)lqLlo, aH = (double)lqH + (double)lqHlo;
     double xd = (aH - aL) * g.rdd + g.offd;
     if (xd < 0.0) xd = 0.0; else if (xd > g.nd - 1 - 1e-6) xd = g.nd - 1 - 1e-6;
     d0 = (int)xd;
@@ -178,8 +213,12 @@ struct ChunkInfo {
     int use_sel;  // sel holds the walked times
     float lw;     // log weight of a random draw
 };
+int exm_tap_parts(const exm_ctx *ctx, int nmc, int nwalk, int rc);
 void exm_run_taps(exm_ctx *ctx, exm_slot &sl, const ChunkInfo &ci, int r0, int rc, bool first_chunk_of_lags);
 void exm_run_gather_planes(exm_ctx *ctx, exm_slot &sl, const ChunkInfo &ci, int r0, int rc);
+void exm_gather_plan(const exm_ctx *ctx, const ChunkInfo &ci, int rc, int *wb, int *ng);
+int exm_gather_parts(const exm_ctx *ctx, int nmc, int m_base, int nwalk, int rc);
+void exm_make_tmap(exm_ctx *ctx, int wb);
 int exm_gather_num_cfgs();
 void exm_run_node_lse(exm_ctx *ctx, exm_slot &sl, int m_base, int nmc);
 void exm_run_lnb(exm_ctx *ctx, exm_slot &sl);

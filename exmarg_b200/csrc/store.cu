@@ -176,14 +176,16 @@ static PFN_cuTensorMapEncodeTiled_v12000 get_encode()
     return fn;
 }
 
-void exm_make_tmap(exm_ctx *ctx)
+// the tensor map of the plane windows of wb rows (kept until the store or the rows change)
+void exm_make_tmap(exm_ctx *ctx, int wb)
 {
+    if (ctx->tmap_ok && ctx->tmap_wb == wb) return;
     // dims innermost first: Delta (ndp), beta (nb), phase plane (nphif), lag (ntau), node (nn)
     cuuint64_t dims[5] = {(cuuint64_t)ctx->ndp, (cuuint64_t)ctx->nb, (cuuint64_t)ctx->nphif, (cuuint64_t)ctx->ntau,
                           (cuuint64_t)ctx->nn};
     const cuuint64_t row = (cuuint64_t)ctx->ndp * exm_dtype_bytes(ctx->dtype);
     cuuint64_t strides[4] = {row, row * ctx->nb, row * ctx->nb * ctx->nphif, row * ctx->nb * ctx->nphif * ctx->ntau};
-    cuuint32_t box[5] = {(cuuint32_t)exm_dtype_wd(ctx->dtype), EXM_WB, 1, 1, 1};
+    cuuint32_t box[5] = {(cuuint32_t)exm_dtype_wd(ctx->dtype), (cuuint32_t)wb, 1, 1, 1};
     cuuint32_t estr[5] = {1, 1, 1, 1, 1};
     const CUtensorMapDataType ty = ctx->dtype == EXM_DTYPE_F32   ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
                                    : ctx->dtype == EXM_DTYPE_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
@@ -193,6 +195,7 @@ void exm_make_tmap(exm_ctx *ctx)
                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) EXM_THROW(EXM_ERR_CUDA, "cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
     ctx->tmap_ok = true;
+    ctx->tmap_wb = wb;
 }
 
 void exm_store_generate(exm_ctx *ctx, int k, const float *M, const float *P, const float *Q, float S, uint32_t seed)
