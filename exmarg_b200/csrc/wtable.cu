@@ -10,12 +10,14 @@
 //   k_w_prep: per quadrature point q, the responses R_I in float32 as the reference forms them (products and
 //             sums rounded one by one; |R| and arg R rounded to float32 from float64), then in float64 the
 //             power ladders m_I^k (k = 0 .. 2 n_max), dph and the damping Bw_j of every node;
+//   k_w_cos:  cos(m dph_q) of every phase class m;
 //   k_w_gemm: for a phase class m the keys form the triangle pw1 = m + 2x, pw2 = m + 2y, x + y <= n_max - m.
-//             A block takes a tile of 8 x-values by 16 y-values (128 keys) and every node (64 rows): a
-//             register-tiled float64 GEMM over q in steps of 16, A[j][q] = Bw_j(q) cos(m dph_q) and
-//             B[q][(x, y)] = m1_q^pw1 m2_q^pw2 formed in shared memory from the 8 + 16 ladder rows of the tile;
-//             the next step's inputs arrive by asynchronous copies (two stages) while a step computes.
+//             A block takes a tile of 8 x-values by 16 y-values (128 keys) and 8 RG rows (nodes): a
+//             register-tiled float64 product over q, A[j][q] = Bw_j(q) and B[q][(x, y)] = m1_q^pw1 (m2_q^pw2
+//             cos(m dph_q)), formed in registers from the tile's 8 + 16 ladder rows; three stages of inputs
+//             arrive by asynchronous copies, one block barrier a step.
 //   k_w_scale: W = Wraw * scale, rounded to float32, non-finite entries counted.
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -23,23 +25,34 @@
 
 namespace {
 
-constexpr int kWRows = 64;       // nodes of a tile (n_nodes <= 64)
+constexpr int kWRows = 64;       // most nodes
 constexpr int kWX = 8;           // powers of |R1| of a tile
 constexpr int kWY = 16;          // powers of |R2| of a tile
 constexpr int kWCols = kWX * kWY;
-constexpr int kWQ = 16;          // quadrature points per step
-constexpr int kWThreads = 128;   // 8 row groups x 16 column groups, 8 x 8 outputs each
+constexpr int kWQ = 32;          // quadrature points per step
+constexpr int kWPitch = kWQ + 2; // of a row in shared memory (doubles): 16-byte rows, two-way conflicts at most
+constexpr int kWStages = 3;
+constexpr int kWThreads = 128;
+
+// quadrature points as stored: rows of a multiple of the step, zero beyond Q (such points add nothing)
+inline int w_pitch(int Q) { return (Q + kWQ - 1) / kWQ * kWQ; }
 
 __global__ void __launch_bounds__(128) k_w_prep(const float *__restrict__ resp, const float *__restrict__ c2p,
                                                 const float *__restrict__ s2p, const float *__restrict__ ap,
                                                 const float *__restrict__ cg, const double *__restrict__ wq, int n_psi,
-                                                int n_chi, int n_nodes, const double *__restrict__ s, int nl,
+                                                int n_chi, int n_nodes, const double *__restrict__ s, int nl, int Qp,
                                                 double *__restrict__ lad1, double *__restrict__ lad2,
                                                 double *__restrict__ dph, double *__restrict__ bw)
 {
     const int Q = n_psi * n_chi;
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= Q) return;
+    if (q >= Qp) return;
+    if (q >= Q) {
+        dph[q] = 0.0;
+        for (int k = 0; k < nl; ++k) lad1[(size_t)k * Qp + q] = lad2[(size_t)k * Qp + q] = 0.0;
+        for (int j = 0; j < n_nodes; ++j) bw[(size_t)j * Qp + q] = 0.0;
+        return;
+    }
     const int ip = q / n_chi, ic = q - ip * n_chi;
     float mag[2], ang[2];
     for (int I = 0; I < 2; ++I) {
@@ -59,106 +72,131 @@ __global__ void __launch_bounds__(128) k_w_prep(const float *__restrict__ resp, 
     for (int k = 1; k < nl; ++k) {
         a1 = __dmul_rn(a1, m1);
         a2 = __dmul_rn(a2, m2);
-        lad1[(size_t)k * Q + q] = a1;
-        lad2[(size_t)k * Q + q] = a2;
+        lad1[(size_t)k * Qp + q] = a1;
+        lad2[(size_t)k * Qp + q] = a2;
     }
     const double w = wq[ic];
     for (int j = 0; j < n_nodes; ++j)
-        bw[(size_t)j * Q + q] = __dmul_rn(exp(-__dadd_rn(__dmul_rn(s[j], S1), __dmul_rn(s[j], S2))), w);
+        bw[(size_t)j * Qp + q] = __dmul_rn(exp(-__dadd_rn(__dmul_rn(s[j], S1), __dmul_rn(s[j], S2))), w);
 }
 
-__device__ __forceinline__ void cp_async8(void *smem, const void *gmem, bool valid)
+// cm[m][q] = cos(m dph_q), once per pixel for all the tiles of a phase class
+__global__ void __launch_bounds__(128) k_w_cos(const double *__restrict__ dph, int Qp, double *__restrict__ cm)
+{
+    const int q = blockIdx.x * blockDim.x + threadIdx.x, m = blockIdx.y;
+    if (q < Qp) cm[(size_t)m * Qp + q] = cos(__dmul_rn((double)m, dph[q]));
+}
+
+__device__ __forceinline__ void cp_async16(void *smem, const void *gmem, bool valid)
 {
     const unsigned dst = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst), "l"(gmem), "r"(valid ? 8 : 0));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(gmem), "r"(valid ? 16 : 0));
 }
 
-__global__ void __launch_bounds__(kWThreads, 2) k_w_gemm(const int4 *__restrict__ tiles, int Q, int n_nodes, int n_max,
+// RG row groups of 8 nodes and QG = 8 / RG groups of threads that share out the quadrature points: thread
+// (tc, rg, qg) holds 8 nodes x 8 keys (x0 + c, y0 + tc) over the points qg, qg + QG, ... of each step, and the
+// point groups' sums are added at the end.  Bound by the float64 pipe: the fewest rows that hold the nodes cost
+// the fewest operations.  Per pixel at order 120: 6 nodes 12.1 ms, 14 nodes 20.5, 30 nodes 38.1, 53 nodes 67.2; one tile
+// of 64 rows with its products staged in shared memory (three barriers a step) took 79 ms whatever the nodes.
+constexpr int w_rows(int rg) { return 8 * rg + kWX + kWY + 1; }
+constexpr size_t w_smem(int rg)
+{
+    const size_t st = sizeof(double) * kWStages * w_rows(rg) * kWPitch;
+    return st > 32768 ? st : 32768;   // at the end: 32 KB of sums to add
+}
+
+template <int RG>
+__global__ void __launch_bounds__(kWThreads, 2) k_w_gemm(const int4 *__restrict__ tiles, int Qp, int n_nodes, int n_max,
                                                          const double *__restrict__ lad1, const double *__restrict__ lad2,
-                                                         const double *__restrict__ dph, const double *__restrict__ bw,
+                                                         const double *__restrict__ cm, const double *__restrict__ bw,
                                                          int t0, double w0, double w1, int n_tau, long long n_keys,
                                                          double *__restrict__ Wraw)
 {
-    // two stages of raw inputs filled by asynchronous copies (the next step's while this one computes)
-    __shared__ double Ar[2][kWQ][kWRows + 1];       // damping rows, then times cos(m dph) in place
-    __shared__ double Ld[2][kWX + kWY][kWQ];        // the tile's |R1| and |R2| ladder rows
-    __shared__ double Dp[2][kWQ];
-    __shared__ double Bs[kWQ][kWCols + 1];
-    __shared__ double cm[kWQ];
+    constexpr int QG = 8 / RG, NR = w_rows(RG);
+    extern __shared__ __align__(16) double wsm[];   // [stage][row: nodes, x ladder, y ladder, cos][point]
     const int4 tl = tiles[blockIdx.x];
     const int m = tl.x, x0 = tl.y, y0 = tl.z;
     const int L = n_max - m + 1;
-    const int tid = threadIdx.x, tr = tid >> 4, tc = tid & 15;
-    const int nsteps = (Q + kWQ - 1) / kWQ;
+    const int tid = threadIdx.x, tc = tid & 15, g = tid >> 4, rg = g % RG, qg = g / RG;
+    const int nsteps = Qp / kWQ;
     auto issue = [&](int step, int buf) {
-        const int q0 = step * kWQ;
-        for (int i = tid; i < kWRows * kWQ; i += kWThreads) {
-            const int row = i >> 4, qq = i & 15, q = q0 + qq;
-            const bool ok = row < n_nodes && q < Q;
-            cp_async8(&Ar[buf][qq][row], ok ? bw + (size_t)row * Q + q : bw, ok);
-        }
-        if (tid < kWQ) {
-            const int q = q0 + tid;
-            cp_async8(&Dp[buf][tid], q < Q ? dph + q : dph, q < Q);
-        } else if (tid < kWQ + (kWX + kWY) * kWQ / 4) {
-            for (int i = (tid - kWQ) * 4; i < (tid - kWQ) * 4 + 4; ++i) {
-                const int row = i / kWQ, qq = i - row * kWQ, q = q0 + qq;
-                if (row < kWX) {
-                    const int x = x0 + row;
-                    const bool ok = x <= L - 1 && q < Q;
-                    cp_async8(&Ld[buf][row][qq], ok ? lad1 + (size_t)(m + 2 * x) * Q + q : lad1, ok);
-                } else {
-                    const int y = y0 + row - kWX;
-                    const bool ok = y <= L - 1 && q < Q;
-                    cp_async8(&Ld[buf][row][qq], ok ? lad2 + (size_t)(m + 2 * y) * Q + q : lad2, ok);
-                }
+        double *st = wsm + (size_t)buf * NR * kWPitch;
+        for (int i = tid; i < NR * (kWQ / 2); i += kWThreads) {
+            const int row = i / (kWQ / 2), qq = 2 * (i - row * (kWQ / 2));
+            const double *src = bw;
+            bool ok;
+            if (row < 8 * RG) {
+                ok = row < n_nodes;
+                if (ok) src = bw + (size_t)row * Qp;
+            } else if (row < 8 * RG + kWX) {
+                const int x = x0 + row - 8 * RG;
+                ok = x <= L - 1;
+                if (ok) src = lad1 + (size_t)(m + 2 * x) * Qp;
+            } else if (row < 8 * RG + kWX + kWY) {
+                const int y = y0 + row - 8 * RG - kWX;
+                ok = y <= L - 1;
+                if (ok) src = lad2 + (size_t)(m + 2 * y) * Qp;
+            } else {
+                ok = true;
+                src = cm + (size_t)m * Qp;
             }
+            cp_async16(st + row * kWPitch + qq, src + (ok ? step * kWQ + qq : 0), ok);
         }
-        asm volatile("cp.async.commit_group;\n" ::);
     };
     double acc[8][8];
 #pragma unroll
     for (int r = 0; r < 8; ++r)
 #pragma unroll
         for (int c = 0; c < 8; ++c) acc[r][c] = 0.0;
-    issue(0, 0);
+#pragma unroll
+    for (int k = 0; k < kWStages - 1; ++k) {
+        if (k < nsteps) issue(k, k);
+        asm volatile("cp.async.commit_group;\n" ::);
+    }
     for (int k = 0; k < nsteps; ++k) {
-        const int buf = k & 1;
-        if (k + 1 < nsteps) issue(k + 1, buf ^ 1);
-        else asm volatile("cp.async.commit_group;\n" ::);
-        asm volatile("cp.async.wait_group 1;\n" ::);
-        __syncthreads();
-        if (tid < kWQ) cm[tid] = (k * kWQ + tid < Q) ? cos(__dmul_rn((double)m, Dp[buf][tid])) : 0.0;
-        __syncthreads();
-        for (int i = tid; i < kWRows * kWQ; i += kWThreads) {
-            const int row = i >> 4, qq = i & 15;
-            Ar[buf][qq][row] = __dmul_rn(Ar[buf][qq][row], cm[qq]);
-        }
-        for (int i = tid; i < kWCols * kWQ; i += kWThreads) {
-            const int c = i >> 4, qq = i & 15;
-            const int x = c >> 4, y = c & 15;   // column c = y + 16 x
-            Bs[qq][c] = __dmul_rn(Ld[buf][x][qq], Ld[buf][kWX + y][qq]);
-        }
-        __syncthreads();
-#pragma unroll 4
-        for (int qq = 0; qq < kWQ; ++qq) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(kWStages - 2));
+        __syncthreads();   // step k has arrived everywhere, and step k - 1's buffer is free
+        if (k + kWStages - 1 < nsteps) issue(k + kWStages - 1, (k + kWStages - 1) % kWStages);
+        asm volatile("cp.async.commit_group;\n" ::);
+        const double *st = wsm + (size_t)(k % kWStages) * NR * kWPitch;
+        const double *pa = st + rg * 8 * kWPitch, *px = st + 8 * RG * kWPitch;
+        const double *py = st + (8 * RG + kWX + tc) * kWPitch, *pc = st + (8 * RG + kWX + kWY) * kWPitch;
+#pragma unroll 2
+        for (int qq = qg; qq < kWQ; qq += QG) {
+            const double yc = __dmul_rn(py[qq], pc[qq]);
             double a[8], b[8];
 #pragma unroll
-            for (int r = 0; r < 8; ++r) a[r] = Ar[buf][qq][tr + 8 * r];
+            for (int r = 0; r < 8; ++r) a[r] = pa[r * kWPitch + qq];
 #pragma unroll
-            for (int c = 0; c < 8; ++c) b[c] = Bs[qq][tc + 16 * c];
+            for (int c = 0; c < 8; ++c) b[c] = __dmul_rn(px[c * kWPitch + qq], yc);
 #pragma unroll
             for (int r = 0; r < 8; ++r)
 #pragma unroll
                 for (int c = 0; c < 8; ++c) acc[r][c] = fma(a[r], b[c], acc[r][c]);
         }
-        __syncthreads();
     }
     asm volatile("cp.async.wait_group 0;\n" ::);
-    // thread (tr, tc) holds rows tr + 8 r and columns tc + 16 c: x = x0 + c, y = y0 + tc
+    // the point groups' sums, halving their number each time
+#pragma unroll
+    for (int h = QG / 2; h > 0; h /= 2) {
+        __syncthreads();
+        double *red = wsm + (size_t)((qg % h) * RG + rg) * 64 * 16 + tc;
+        if (qg >= h && qg < 2 * h)
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+#pragma unroll
+                for (int c = 0; c < 8; ++c) red[(r * 8 + c) * 16] = acc[r][c];
+        __syncthreads();
+        if (qg < h)
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+#pragma unroll
+                for (int c = 0; c < 8; ++c) acc[r][c] = __dadd_rn(acc[r][c], red[(r * 8 + c) * 16]);
+    }
+    if (qg) return;
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
-        const int row = tr + 8 * r;
+        const int row = rg * 8 + r;
         if (row >= n_nodes) continue;
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
@@ -203,7 +241,7 @@ extern "C" int exm_w_build(exm_ctx *ctx, int n_nodes, const double *s_nodes, int
             EXM_THROW(EXM_ERR_ARG, "null argument");
         for (int p = 0; p < n_pix; ++p)
             if (j0[p] < 0 || j0[p] > n_tau - 2) EXM_THROW(EXM_ERR_ARG, "delay bin outside the tau grid");
-        const int Q = n_psi * n_chi, nl = 2 * n_max + 1;
+        const int Q = n_psi * n_chi, Qp = w_pitch(Q), nl = 2 * n_max + 1;
         const long long n_keys = (long long)(n_max + 1) * (n_max + 2) * (n_max + 3) / 6;
         std::vector<int4> tiles;
         for (int m = 0; m <= n_max; ++m) {
@@ -212,7 +250,7 @@ extern "C" int exm_w_build(exm_ctx *ctx, int n_nodes, const double *s_nodes, int
                 for (int y0 = 0; x0 + y0 <= L - 1; y0 += kWY) tiles.push_back(make_int4(m, x0, y0, 0));
         }
         const size_t nW = (size_t)n_nodes * n_tau * n_keys;
-        dbuf d_s, d_c2p, d_s2p, d_ap, d_cg, d_wq, d_resp, d_scale, d_W, d_out, d_tiles, d_l1, d_l2, d_dph, d_bw, d_bad;
+        dbuf d_s, d_c2p, d_s2p, d_ap, d_cg, d_wq, d_resp, d_scale, d_W, d_out, d_tiles, d_l1, d_l2, d_dph, d_cm, d_bw, d_bad;
         struct Guard {
             exm_ctx *c;
             std::vector<dbuf *> b;
@@ -222,7 +260,7 @@ extern "C" int exm_w_build(exm_ctx *ctx, int n_nodes, const double *s_nodes, int
                     if (x->p) exm_free(c, *x);
             }
         } guard{ctx, {&d_s, &d_c2p, &d_s2p, &d_ap, &d_cg, &d_wq, &d_resp, &d_scale, &d_W, &d_out, &d_tiles, &d_l1,
-                      &d_l2, &d_dph, &d_bw, &d_bad}};
+                      &d_l2, &d_dph, &d_cm, &d_bw, &d_bad}};
         auto up = [&](dbuf &b, const void *src, size_t bytes) {
             exm_alloc(ctx, b, bytes);
             EXM_CUDA(cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
@@ -238,10 +276,11 @@ extern "C" int exm_w_build(exm_ctx *ctx, int n_nodes, const double *s_nodes, int
         up(d_tiles, tiles.data(), tiles.size() * sizeof(int4));
         exm_alloc(ctx, d_W, nW * sizeof(double));
         exm_alloc(ctx, d_out, nW * sizeof(float));
-        exm_alloc(ctx, d_l1, (size_t)nl * Q * sizeof(double));
-        exm_alloc(ctx, d_l2, (size_t)nl * Q * sizeof(double));
-        exm_alloc(ctx, d_dph, (size_t)Q * sizeof(double));
-        exm_alloc(ctx, d_bw, (size_t)n_nodes * Q * sizeof(double));
+        exm_alloc(ctx, d_l1, (size_t)nl * Qp * sizeof(double));
+        exm_alloc(ctx, d_l2, (size_t)nl * Qp * sizeof(double));
+        exm_alloc(ctx, d_dph, (size_t)Qp * sizeof(double));
+        exm_alloc(ctx, d_cm, (size_t)(n_max + 1) * Qp * sizeof(double));
+        exm_alloc(ctx, d_bw, (size_t)n_nodes * Qp * sizeof(double));
         exm_alloc(ctx, d_bad, sizeof(unsigned long long));
         EXM_CUDA(cudaMemsetAsync(d_W.p, 0, nW * sizeof(double), ctx->stream));
         EXM_CUDA(cudaMemsetAsync(d_bad.p, 0, sizeof(unsigned long long), ctx->stream));
@@ -250,17 +289,32 @@ extern "C" int exm_w_build(exm_ctx *ctx, int n_nodes, const double *s_nodes, int
         EXM_CUDA(cudaEventCreate(&e1));
         EXM_CUDA(cudaEventCreate(&e2));
         EXM_CUDA(cudaEventRecord(e0, ctx->stream));
-        for (int p = 0; p < n_pix; ++p) {
-            k_w_prep<<<(Q + 127) / 128, 128, 0, ctx->stream>>>((const float *)d_resp.p + 4 * (size_t)p,
-                                                               (const float *)d_c2p.p, (const float *)d_s2p.p,
-                                                               (const float *)d_ap.p, (const float *)d_cg.p,
-                                                               (const double *)d_wq.p, n_psi, n_chi, n_nodes,
-                                                               (const double *)d_s.p, nl, (double *)d_l1.p,
-                                                               (double *)d_l2.p, (double *)d_dph.p, (double *)d_bw.p);
-            k_w_gemm<<<(int)tiles.size(), kWThreads, 0, ctx->stream>>>(
-                (const int4 *)d_tiles.p, Q, n_nodes, n_max, (const double *)d_l1.p, (const double *)d_l2.p,
-                (const double *)d_dph.p, (const double *)d_bw.p, j0[p], w[2 * p], w[2 * p + 1], n_tau, n_keys,
+        auto gemm = [&](auto rg, int p) {
+            constexpr int RG = decltype(rg)::value;
+            exm_allow_smem(ctx, (const void *)k_w_gemm<RG>, w_smem(RG));
+            k_w_gemm<RG><<<(int)tiles.size(), kWThreads, w_smem(RG), ctx->stream>>>(
+                (const int4 *)d_tiles.p, Qp, n_nodes, n_max, (const double *)d_l1.p, (const double *)d_l2.p,
+                (const double *)d_cm.p, (const double *)d_bw.p, j0[p], w[2 * p], w[2 * p + 1], n_tau, n_keys,
                 (double *)d_W.p);
+        };
+        for (int p = 0; p < n_pix; ++p) {
+            k_w_prep<<<(Qp + 127) / 128, 128, 0, ctx->stream>>>((const float *)d_resp.p + 4 * (size_t)p,
+                                                                (const float *)d_c2p.p, (const float *)d_s2p.p,
+                                                                (const float *)d_ap.p, (const float *)d_cg.p,
+                                                                (const double *)d_wq.p, n_psi, n_chi, n_nodes,
+                                                                (const double *)d_s.p, nl, Qp, (double *)d_l1.p,
+                                                                (double *)d_l2.p, (double *)d_dph.p, (double *)d_bw.p);
+            k_w_cos<<<dim3((Qp + 127) / 128, n_max + 1), 128, 0, ctx->stream>>>((const double *)d_dph.p, Qp,
+                                                                               (double *)d_cm.p);
+            // the fewest rows that hold the nodes
+            if (n_nodes <= 8)
+                gemm(std::integral_constant<int, 1>(), p);
+            else if (n_nodes <= 16)
+                gemm(std::integral_constant<int, 2>(), p);
+            else if (n_nodes <= 32)
+                gemm(std::integral_constant<int, 4>(), p);
+            else
+                gemm(std::integral_constant<int, 8>(), p);
         }
         EXM_CUDA(cudaGetLastError());
         EXM_CUDA(cudaEventRecord(e1, ctx->stream));
@@ -284,7 +338,7 @@ extern "C" int exm_w_build(exm_ctx *ctx, int n_nodes, const double *s_nodes, int
             ms_out[0] = k_ms;
             ms_out[1] = all_ms;
         }
-        ctx->launches += 2 * n_pix + 1;
+        ctx->launches += 3 * n_pix + 1;
     } catch (const exm_error &e) {
         ctx->err = e.msg;
         return e.code;
