@@ -9,7 +9,7 @@
 // k_rs_surf: one block per template: its finite (y, ln Lambda) points sorted by y in shared memory,
 //            then every z of the grid.
 // k_rs_out:  one block per z: the templates finite at that z (a block-wide scan), then every m1.
-// k_rs_lnb:  one block: the log of the weighted mean, max then sum.
+// k_rs_lnb_part, k_rs_lnb: the log of the weighted mean, max then sum, over parts of the grid and over the parts.
 #include <cmath>
 
 #include "common.cuh"
@@ -18,7 +18,7 @@
 struct exm_redshift {
     int nn1 = 0, nm = 0, nz = 0, nm1 = 0;
     dbuf yN, M, yq, z, m1, w;   // [nn1][nm], [nm], [nz], [nz], [nm1], [nm1][nz]
-    dbuf lamN, surf, out, red;  // [nn1][nm], [nz][nm], [nm1][nz], 2 doubles
+    dbuf lamN, surf, out, red;  // [nn1][nm], [nz][nm], [nm1][nz], ln B and the (max, sum) of its parts
 };
 
 #define EXM_RS_MAX_POINTS (EXM_MAX_NODES + 1)
@@ -125,38 +125,66 @@ __global__ void __launch_bounds__(256) k_rs_out(const double *__restrict__ surf,
     }
 }
 
-// ln sum_i w_i exp(L_i) over the finite L with w > 0 (exmarg/search/pe.py:135-142); red[0] = ln B
-__global__ void __launch_bounds__(1024) k_rs_lnb(const double *__restrict__ L, const double *__restrict__ w,
-                                                 long long n, double *__restrict__ red)
+// ln sum_i w_i exp(L_i) over the finite L with w > 0 (exmarg/search/pe.py:135-142), in two steps: each block
+// the maximum and the sum relative to it of its share of the grid, then one block over those.  (One block
+// over the whole grid took 1.7 ms on 1600 x 1600: one SM's loads and float64 exponentials.)
+#define EXM_RS_PARTS 592
+
+__device__ __forceinline__ double rs_block_max(double v, double *sh)
 {
-    __shared__ double sh[32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    if (lane == 0) sh[warp] = v;
+    __syncthreads();
+    for (int q = 0; q < nw; ++q) v = fmax(v, sh[q]);
+    __syncthreads();
+    return v;
+}
+
+__device__ __forceinline__ double rs_block_sum(double v, double *sh)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) sh[warp] = v;
+    __syncthreads();
+    v = 0.0;
+    for (int q = 0; q < nw; ++q) v += sh[q];
+    __syncthreads();
+    return v;
+}
+
+__global__ void __launch_bounds__(256) k_rs_lnb_part(const double *__restrict__ L, const double *__restrict__ w,
+                                                     long long n, double *__restrict__ part)
+{
+    __shared__ double sh[8];
+    const long long a = n * blockIdx.x / gridDim.x, b = n * (blockIdx.x + 1) / gridDim.x;
     double mx = -INFINITY;
-    for (long long i = threadIdx.x; i < n; i += blockDim.x)
+    for (long long i = a + threadIdx.x; i < b; i += blockDim.x)
         if (isfinite(L[i]) && w[i] > 0.0) mx = fmax(mx, L[i]);
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) sh[warp] = mx;
-    __syncthreads();
-    if (warp == 0) {
-        double v = lane < (int)(blockDim.x >> 5) ? sh[lane] : -INFINITY;
-        for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-        if (lane == 0) sh[0] = v;
-    }
-    __syncthreads();
-    mx = sh[0];
-    __syncthreads();
+    mx = rs_block_max(mx, sh);
     double acc = 0.0;
     if (isfinite(mx))
-        for (long long i = threadIdx.x; i < n; i += blockDim.x)
+        for (long long i = a + threadIdx.x; i < b; i += blockDim.x)
             if (isfinite(L[i]) && w[i] > 0.0) acc += w[i] * exp(L[i] - mx);
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) sh[warp] = acc;
-    __syncthreads();
+    acc = rs_block_sum(acc, sh);
     if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int q = 0; q < (int)(blockDim.x >> 5); ++q) t += sh[q];
-        red[0] = isfinite(mx) ? mx + log(t) : -INFINITY;
+        part[2 * blockIdx.x] = mx;
+        part[2 * blockIdx.x + 1] = acc;
     }
+}
+
+__global__ void __launch_bounds__(256) k_rs_lnb(const double *__restrict__ part, int n, double *__restrict__ out)
+{
+    __shared__ double sh[8];
+    double mx = -INFINITY;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) mx = fmax(mx, part[2 * i]);
+    mx = rs_block_max(mx, sh);
+    double acc = 0.0;
+    if (isfinite(mx))
+        for (int i = threadIdx.x; i < n; i += blockDim.x)
+            if (isfinite(part[2 * i])) acc += part[2 * i + 1] * exp(part[2 * i] - mx);
+    acc = rs_block_sum(acc, sh);
+    if (threadIdx.x == 0) out[0] = isfinite(mx) ? mx + log(acc) : -INFINITY;
 }
 
 void exm_redshift_release(exm_ctx *ctx)
@@ -201,7 +229,7 @@ extern "C" int exm_redshift_grid(exm_ctx *ctx, int nn1, int nm, const double *yN
         exm_alloc(ctx, r->lamN, sizeof(double) * nn1 * nm);
         exm_alloc(ctx, r->surf, sizeof(double) * (size_t)nz * nm);
         exm_alloc(ctx, r->out, sizeof(double) * (size_t)nm1 * nz);
-        exm_alloc(ctx, r->red, 2 * sizeof(double));
+        exm_alloc(ctx, r->red, (2 + 2 * EXM_RS_PARTS) * sizeof(double));
         exm_allow_smem(ctx, (const void *)k_rs_out, 2 * sizeof(int) * (size_t)nm);
         EXM_CUDA(cudaStreamSynchronize(ctx->stream));
     } catch (const exm_error &e) {
@@ -232,10 +260,13 @@ extern "C" int exm_source_frame(exm_ctx *ctx, const double *lamN, double *ln_lam
         k_rs_out<<<r->nz, 256, 2 * sizeof(int) * (size_t)r->nm, ctx->stream>>>(
             (const double *)r->surf.p, r->nm, (const double *)r->M.p, (const double *)r->z.p, r->nz,
             (const double *)r->m1.p, r->nm1, (double *)r->out.p);
-        k_rs_lnb<<<1, 1024, 0, ctx->stream>>>((const double *)r->out.p, (const double *)r->w.p,
-                                              (long long)r->nm1 * r->nz, (double *)r->red.p);
+        double *part = (double *)r->red.p + 2;
+        const long long cells = (long long)r->nm1 * r->nz;
+        const int parts = (int)std::min<long long>(EXM_RS_PARTS, (cells + 1023) / 1024);
+        k_rs_lnb_part<<<parts, 256, 0, ctx->stream>>>((const double *)r->out.p, (const double *)r->w.p, cells, part);
+        k_rs_lnb<<<1, 256, 0, ctx->stream>>>(part, parts, (double *)r->red.p);
         EXM_CUDA(cudaGetLastError());
-        ctx->launches += 3;
+        ctx->launches += 4;
         if (ln_lambda_out)
             EXM_CUDA(cudaMemcpyAsync(ln_lambda_out, r->out.p, sizeof(double) * (size_t)r->nm1 * r->nz,
                                      cudaMemcpyDeviceToHost, ctx->stream));
