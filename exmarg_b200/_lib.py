@@ -504,10 +504,14 @@ class Context:
                                                _p(z), m1.size, _p(m1), _p(w)))
         self.rs_shape = (m1.size, z.size)
 
-    def source_frame(self, lamN, want=True):
-        """(ln_lambda (nm1, nz) or None, ln_b) of one segment's node values"""
+    def source_frame(self, lamN, want=True, out=None):
+        """(ln_lambda (nm1, nz) or None, ln_b) of one segment's node values; out: a C-ordered float64 array of that
+        shape to write ln_lambda into"""
         lamN = np.ascontiguousarray(lamN, np.float64)
-        out = np.empty(self.rs_shape, np.float64) if want else None
+        if out is None:
+            out = np.empty(self.rs_shape, np.float64) if want else None
+        elif out.shape != tuple(self.rs_shape) or out.dtype != np.float64 or not out.flags.c_contiguous:
+            raise ValueError("out must be a C-ordered float64 array of the grid's shape")
         lnb = np.zeros(1, np.float64)
         self._check(self.lib.exm_source_frame(self.h, _p(lamN), _p(out), _p(lnb)))
         return out, float(lnb[0])

@@ -352,6 +352,7 @@ static void ctx_free(exm_ctx *ctx)
 {
     cudaSetDevice(ctx->dev);
     cudaStreamSynchronize(ctx->stream);
+    exm_hostio_release(ctx);
     exm_redshift_release(ctx);
     if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
     if (ctx->plan) cufftDestroy(ctx->plan);
@@ -1253,27 +1254,15 @@ extern "C" int exm_filter(exm_ctx *ctx, const double *d_H, const double *d_L, co
     ensure_slot(ctx, sl, rs);
     stage_input(ctx, sl, d_H, d_L, sig2_H, sig2_L);
     exm_run_filter(ctx, sl, (const float2 *)ctx->d_W.p, ctx->nm);
+    if (traj_out) {   // laid out on the device (the transforms' buffer is free now), then one copy
+        exm_run_traj_planes(ctx, sl, (float *)sl.desc.p, true);
+        exm_copy_out(ctx, traj_out, sl.desc.p, 4 * (size_t)ctx->nm * ctx->nt * sizeof(float));
+    }
     EXM_CUDA(cudaStreamSynchronize(ctx->stream));
     ctx->traj_ok = true;
     ctx->times_ok = false;
     ctx->cur_nwalk = ctx->nt;
     ctx->cur_lw = 0.f;
-    if (traj_out) {
-        const size_t nt = ctx->nt, nm = ctx->nm;
-        std::vector<float2> h(2 * nm * nt);
-        EXM_CUDA(cudaMemcpy(h.data(), sl.traj.p, sizeof(float2) * h.size(), cudaMemcpyDeviceToHost));
-        for (int det = 0; det < 2; ++det)
-            for (size_t i = 0; i < nm; ++i) {
-                const size_t m = ctx->order[i];
-                const float2 *src = &h[(det * nm + i) * nt];
-                float *lq = traj_out + ((size_t)(2 * det) * nm + m) * nt;
-                float *ph = traj_out + ((size_t)(2 * det + 1) * nm + m) * nt;
-                for (size_t t = 0; t < nt; ++t) {
-                    lq[t] = src[t].x;
-                    ph[t] = src[t].y;
-                }
-            }
-    }
     API_END(ctx)
 }
 
@@ -1285,19 +1274,12 @@ extern "C" int exm_set_trajectories(exm_ctx *ctx, const float *traj)
     RunShape rs = stage_shape(ctx, 0, 0);
     exm_slot &sl = ctx->slot;
     ensure_slot(ctx, sl, rs);
-    const size_t nt = ctx->nt, nm = ctx->nm;
-    std::vector<float2> h(2 * nm * nt);
-    for (int det = 0; det < 2; ++det)
-        for (size_t i = 0; i < nm; ++i) {
-            const size_t m = ctx->order[i];
-            const float *lq = traj + ((size_t)(2 * det) * nm + m) * nt;
-            const float *ph = traj + ((size_t)(2 * det + 1) * nm + m) * nt;
-            float2 *dst = &h[(det * nm + i) * nt];
-            for (size_t t = 0; t < nt; ++t) dst[t] = make_float2(lq[t], ph[t]);
-        }
-    EXM_CUDA(cudaMemcpy(sl.traj.p, h.data(), sizeof(float2) * h.size(), cudaMemcpyHostToDevice));
+    const size_t n = (size_t)ctx->nm * ctx->nt;
+    exm_copy_in(ctx, sl.desc.p, traj, 4 * n * sizeof(float));
+    exm_run_traj_planes(ctx, sl, (float *)sl.desc.p, false);
     if (sl.trajlo.p)   // float32 trajectories: no residual
-        EXM_CUDA(cudaMemset(sl.trajlo.p, 0, std::min(sl.trajlo.bytes, sizeof(float) * h.size())));
+        EXM_CUDA(cudaMemsetAsync(sl.trajlo.p, 0, std::min(sl.trajlo.bytes, 2 * n * sizeof(float)), ctx->stream));
+    EXM_CUDA(cudaStreamSynchronize(ctx->stream));
     ctx->traj_ok = true;
     ctx->times_ok = false;
     ctx->cur_nwalk = ctx->nt;

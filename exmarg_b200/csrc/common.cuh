@@ -46,6 +46,7 @@ struct exm_error {
 
 struct exm_ctx;
 struct exm_server;   // the native request loop of a context (serve.cu)
+struct exm_hostio;   // pinned slots for large copies (hostio.cu)
 
 struct dbuf {
     void *p = nullptr;
@@ -152,6 +153,7 @@ struct exm_ctx {
     dbuf d_stats;                     // uint64 [4]: gather counters (slow-path taps, boundary taps)
 
     // launch shape of the plane gather (index into its table; chosen by exm_autotune)
+    exm_hostio *hostio = nullptr;        // made by the first large copy from or to pageable memory
     struct exm_redshift *rs = nullptr;   // pe_redshift's grid and buffers (csrc/redshift.cu)
     int gather_cfg = 0;
     int gather_chunk_pct = 150;

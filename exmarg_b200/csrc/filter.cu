@@ -61,6 +61,33 @@ __global__ void k_polar(const double2 *__restrict__ z, float2 *__restrict__ out,
     }
 }
 
+// the trajectories between their float2 pairs (internal template order) and the four float planes lqH, phH, lqL,
+// phL of the host's layout (bank order)
+__global__ void k_traj_planes(float2 *__restrict__ traj, float *__restrict__ planes, const int *__restrict__ order, int nm,
+                              int nt, int out)
+{
+    const int i = blockIdx.y % nm, det = blockIdx.y / nm;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nt) return;
+    float2 *p = traj + ((long long)det * nm + i) * nt + t;
+    float *lq = planes + ((long long)(2 * det) * nm + order[i]) * nt + t, *ph = lq + (long long)nm * nt;
+    if (out) {
+        const float2 v = *p;
+        *lq = v.x;
+        *ph = v.y;
+    } else {
+        *p = make_float2(*lq, *ph);
+    }
+}
+
+void exm_run_traj_planes(exm_ctx *ctx, exm_slot &sl, float *planes, bool out)
+{
+    k_traj_planes<<<dim3((ctx->nt + 255) / 256, 2 * ctx->nm), 256, 0, ctx->stream>>>(
+        (float2 *)sl.traj.p, planes, (const int *)ctx->d_order.p, ctx->nm, ctx->nt, out ? 1 : 0);
+    EXM_CUDA(cudaGetLastError());
+    ctx->launches += 1;
+}
+
 void exm_run_filter(exm_ctx *ctx, exm_slot &sl, const float2 *dW, int nm)
 {
     const int nt = ctx->nt, nf = ctx->nfreq;

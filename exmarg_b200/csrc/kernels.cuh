@@ -198,6 +198,10 @@ void exm_store_quantize(exm_ctx *ctx, int k, const float *src, int sp);
 void exm_store_load_run(exm_ctx *ctx, int first, int n, const char *const *paths, const int64_t *offsets,
                         const float *const *hosts, int readers, long long chunk_bytes, int flags, double *stats);
 void exm_redshift_release(exm_ctx *ctx);
+void exm_hostio_release(exm_ctx *ctx);
+void exm_copy_out(exm_ctx *ctx, void *host, const void *dev, size_t bytes);
+void exm_copy_in(exm_ctx *ctx, void *dev, const void *host, size_t bytes);
+void exm_run_traj_planes(exm_ctx *ctx, exm_slot &sl, float *planes, bool out);
 void exm_store_dequantize(exm_ctx *ctx, int k, float *dst, int dp);
 
 void exm_fft_plan(exm_ctx *ctx, int batch);

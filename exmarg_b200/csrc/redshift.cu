@@ -268,8 +268,7 @@ extern "C" int exm_source_frame(exm_ctx *ctx, const double *lamN, double *ln_lam
         EXM_CUDA(cudaGetLastError());
         ctx->launches += 4;
         if (ln_lambda_out)
-            EXM_CUDA(cudaMemcpyAsync(ln_lambda_out, r->out.p, sizeof(double) * (size_t)r->nm1 * r->nz,
-                                     cudaMemcpyDeviceToHost, ctx->stream));
+            exm_copy_out(ctx, ln_lambda_out, r->out.p, sizeof(double) * (size_t)r->nm1 * r->nz);
         double lnb = 0.0;
         EXM_CUDA(cudaMemcpyAsync(&lnb, r->red.p, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
         EXM_CUDA(cudaStreamSynchronize(ctx->stream));

@@ -201,7 +201,7 @@ extern "C" int exm_k_edges(exm_ctx *ctx, int n_max, int n_tau, const double *Wd,
         } guard{ctx, {&dW, &dco, &dlnq, &dgmo, &dcos, &dcls, &dcls0, &dC, &dcol, &drow}};
         auto up = [&](dbuf &b, const void *src, size_t bytes) {
             exm_alloc(ctx, b, bytes);
-            EXM_CUDA(cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
+            exm_copy_in(ctx, b.p, src, bytes);
         };
         cudaEvent_t e0, e1;
         EXM_CUDA(cudaEventCreate(&e0));
@@ -225,8 +225,8 @@ extern "C" int exm_k_edges(exm_ctx *ctx, int n_max, int n_tau, const double *Wd,
                                                                 (const double *)dgmo.p, (float *)dcol.p, (float *)drow.p);
         EXM_CUDA(cudaGetLastError());
         EXM_CUDA(cudaEventRecord(e1, ctx->stream));
-        EXM_CUDA(cudaMemcpyAsync(col_out, dcol.p, nE * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
-        EXM_CUDA(cudaMemcpyAsync(row_out, drow.p, nE * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
+        exm_copy_out(ctx, col_out, dcol.p, nE * sizeof(float));
+        exm_copy_out(ctx, row_out, drow.p, nE * sizeof(float));
         EXM_CUDA(cudaStreamSynchronize(ctx->stream));
         float k_ms = 0.f;
         cudaEventElapsedTime(&k_ms, e0, e1);
@@ -284,8 +284,8 @@ extern "C" int exm_bd_build(exm_ctx *ctx, int nord, int ntau, int nq, int nphif,
         EXM_CUDA(cudaEventCreate(&e2));
         EXM_CUDA(cudaEventCreate(&e3));
         EXM_CUDA(cudaEventRecord(e0, ctx->stream));
-        EXM_CUDA(cudaMemcpyAsync(dcol.p, col, nin * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
-        EXM_CUDA(cudaMemcpyAsync(drow.p, row, nin * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
+        exm_copy_in(ctx, dcol.p, col, nin * sizeof(float));
+        exm_copy_in(ctx, drow.p, row, nin * sizeof(float));
         EXM_CUDA(cudaMemcpyAsync(dlnq.p, lnq, nq * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
         EXM_CUDA(cudaMemcpyAsync(dbeta.p, beta, nb * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
         EXM_CUDA(cudaMemcpyAsync(dlad.p, ladder, n_ladder * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
@@ -302,8 +302,7 @@ extern "C" int exm_bd_build(exm_ctx *ctx, int nord, int ntau, int nq, int nphif,
         EXM_CUDA(cudaGetLastError());
         EXM_CUDA(cudaEventRecord(e2, ctx->stream));
         unsigned long long bad = 0;
-        EXM_CUDA(cudaMemcpyAsync(T_out, dT.p, (size_t)n_ladder * per * sizeof(float), cudaMemcpyDeviceToHost,
-                                 ctx->stream));
+        exm_copy_out(ctx, T_out, dT.p, (size_t)n_ladder * per * sizeof(float));
         EXM_CUDA(cudaMemcpyAsync(&bad, dbad.p, sizeof(bad), cudaMemcpyDeviceToHost, ctx->stream));
         EXM_CUDA(cudaEventRecord(e3, ctx->stream));
         EXM_CUDA(cudaStreamSynchronize(ctx->stream));

@@ -263,7 +263,7 @@ extern "C" int exm_w_build(exm_ctx *ctx, int n_nodes, const double *s_nodes, int
                       &d_l2, &d_dph, &d_cm, &d_bw, &d_bad}};
         auto up = [&](dbuf &b, const void *src, size_t bytes) {
             exm_alloc(ctx, b, bytes);
-            EXM_CUDA(cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
+            exm_copy_in(ctx, b.p, src, bytes);
         };
         up(d_s, s_nodes, n_nodes * sizeof(double));
         up(d_c2p, c2p, n_psi * sizeof(float));
@@ -323,7 +323,7 @@ extern "C" int exm_w_build(exm_ctx *ctx, int n_nodes, const double *s_nodes, int
                                                               (unsigned long long *)d_bad.p);
         EXM_CUDA(cudaGetLastError());
         unsigned long long bad = 0;
-        EXM_CUDA(cudaMemcpyAsync(W_out, d_out.p, nW * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
+        exm_copy_out(ctx, W_out, d_out.p, nW * sizeof(float));
         EXM_CUDA(cudaMemcpyAsync(&bad, d_bad.p, sizeof(bad), cudaMemcpyDeviceToHost, ctx->stream));
         EXM_CUDA(cudaEventRecord(e2, ctx->stream));
         EXM_CUDA(cudaStreamSynchronize(ctx->stream));

@@ -247,7 +247,7 @@ def pe_redshift(segments, bank, store, rows=None, chunk=8, zmax=8.0, nz=1600, m1
         ctx.redshift_grid(_node_y(store, np.asarray(bank.u, float), ymin), M, D0 / dl, z, m1, w)
         ctx.rs_key = key
     nn = len(store.s)
-    out = np.full((seg["rows"].size, m1.size, z.size), -np.inf)
+    out = np.empty((seg["rows"].size, m1.size, z.size))
     ln_b = np.empty(seg["rows"].size)
     for e, row in enumerate(seg["rows"]):
         ctx.filter(seg["d_H"][e:e + 1], seg["d_L"][e:e + 1], seg["sig2_H"], seg["sig2_L"], want=False)
@@ -256,5 +256,5 @@ def pe_redshift(segments, bank, store, rows=None, chunk=8, zmax=8.0, nz=1600, m1
         else:
             ctx.set_times(None)
         lamN = ctx.node_values(nn)
-        out[e], ln_b[e] = ctx.source_frame(lamN)
+        _, ln_b[e] = ctx.source_frame(lamN, out=out[e])
     return dict(m1=m1, z=z, ln_lambda=out, ln_b=ln_b, rows=seg["rows"])

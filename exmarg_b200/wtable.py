@@ -127,10 +127,10 @@ def keys(n_max):
 def scales(s_nodes, n_max):
     """(n_nodes, n_keys) s^n / n! 2^n, its logarithm capped at 700 (w_gpu.py:146-151)"""
     from scipy.special import gammaln
-    n_key = np.array([k[0] for k in keys(n_max)], float)
+    n = np.arange(n_max + 1, dtype=float)   # the scale depends on a key's order alone: (n + 1)(n + 2) / 2 keys of order n
     s = np.atleast_1d(np.asarray(s_nodes, float))
-    ln_scale = n_key[None, :] * np.log(s)[:, None] - gammaln(n_key + 1.0)[None, :] + n_key[None, :] * np.log(2.0)
-    return np.exp(np.minimum(ln_scale, 700.0))
+    ln_scale = n[None, :] * np.log(s)[:, None] - gammaln(n + 1.0)[None, :] + n[None, :] * np.log(2.0)
+    return np.repeat(np.exp(np.minimum(ln_scale, 700.0)), [(k + 1) * (k + 2) // 2 for k in range(n_max + 1)], axis=1)
 
 
 def geometry(nside, n_max, n_tau, pixels=None):
