@@ -14,15 +14,16 @@
 // path that reads the table from global memory.
 //
 // What bounds it (2048 templates x 53 nodes x 87 lags x 2048 times, 1.65e10 taps): shared-memory reads (eight a
-// tap, 69 % of the data pipe) and instruction issue (61 %) together; DRAM is at a tenth of its rate.  92.7 -> 65.3 ms:
+// tap, 69 % of the data pipe) and instruction issue (61 %) together; DRAM is at a tenth of its rate.  92.7 -> 62.7 ms:
 //  * four taps of one template per group: the bookkeeping of templates, the ranges and the running maximum are paid
-//    once for four taps (5.4 -> 2.9 warp instructions per tap); padding the runs to whole groups adds 3.8 % taps;
+//    once for four taps (5.4 -> 2.8 warp instructions per tap); padding the runs to whole groups adds 3.8 % taps;
 //  * a row pitch of a multiple of the 32 banks, and taps ordered so that a step's lanes hit different banks
 //    (k_tap_order): 3.4 -> 2.4 cycles per read;
 //  * boundary points in blocks of their own, so the accumulators take 24 instead of 80 bytes a template and a block
 //    takes 1024 templates: every plane pair costs a block a fixed ~6 us of waits (68.0 at 704, 75.5 at 352);
 //  * a warp's first descriptors and end templates of the next pair loaded before it waits for that pair's planes.
-// 20 warps at 96 registers: 16 warps 68.5 ms (too few to cover the latencies), 24 and 28 spill (67.0, 80.4).
+//  * descriptors loaded by whole chunks: no lane's loads are predicated or replaced by constants (65.3 -> 62.7).
+// 20 warps at 96 registers: 16 warps 64.2 ms (too few to cover the latencies), 24 and 28 spill (68.4, 80).
 //
 // k_gather_simple (the gather_cpu / gather_gpu contract, any table per slot): one
 // block per (row, lag), the reference's arithmetic in float64.
@@ -247,25 +248,29 @@ struct RunCtx {
     int tF, tL;                 // the templates at the two ends of this warp's taps (may be shared with
     unsigned eF, eL;            // neighbouring warps): their partials go to this warp's edge slots (m, S)
     unsigned q, qn;             // this warp's queue of exact-path taps for the pair (int2 entries) and its count
-    // the lane's next group of descriptors: whether it lies in [beg, end), its first position, its address,
-    // its index in the chunk
+    // the lane's next group of descriptors: whether it lies in [beg, end), its first position, its chunk's, its
+    // index in the chunk, its address
     uint4 nx[EXM_GT];
     bool in;
-    int jl, gn;
+    int jl, jc, gn;
     const uint4 *pn;
 };
 
-// load the lane's next group and step to the one after
+// load the lane's next group and step to the one after.  A lane whose group lies outside [beg, end) loads what is
+// stored there (its chunk is a chunk of the run) and discards it by `in`; a chunk past the run's last is not read.
 __device__ __forceinline__ void next_group(RunCtx &c)
 {
     c.in = c.jl >= c.beg && c.jl < c.end;
+    if (c.jc < c.end) {
 #pragma unroll
-    for (int u = 0; u < EXM_GT; ++u) c.nx[u] = c.in ? __ldg(c.pn + 32 * u) : make_uint4(0u, 0u, 0u, EXM_DESC_PAD);
+        for (int u = 0; u < EXM_GT; ++u) c.nx[u] = __ldg(c.pn + 32 * u);
+    }
     c.pn += 32 * EXM_GT;
     c.jl += EXM_GT;
     if (++c.gn == c.ng) {   // on to the next chunk
         c.gn = 0;
         c.jl += EXM_GT * 31 * c.ng;
+        c.jc += EXM_GT * 32 * c.ng;
     }
 }
 
@@ -381,6 +386,7 @@ __device__ __forceinline__ void open_share(RunCtx &c, int beg, int end, int pair
     if (c.beg < c.end) {
         const int jstart = c.beg & ~(ch - 1);
         c.gn = 0;
+        c.jc = jstart;
         c.jl = jstart + EXM_GT * c.ng * lane;
         c.pn = c.descr + jstart + lane;
         next_group(c);
