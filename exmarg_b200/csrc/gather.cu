@@ -907,7 +907,8 @@ static int planes_tch(const exm_ctx *ctx, const ChunkInfo &ci, int rc, int pct, 
 // The windows' height and the descriptors' chunk, which the tap build and the gather share.  Rows: the most that
 // fit beside the accumulators of the templates a default block takes (at least EXM_WB_MIN, at most
 // EXM_WB_MAX): every row more leaves fewer taps to the exact path.  Groups per lane: 4 (chunks of 512 taps),
-// fewer when a plane pair of a block has too few taps to give every warp a chunk.
+// fewer when a plane pair of a block has too few taps to give every warp a chunk (gather ms at 4 / 2 / 1 groups:
+// 10900 taps 10.6 / 11.2 / 12.9, 8000 7.8 / 7.8 / 8.8, 5100 7.3 / 6.7 / 7.4, 2700 0.45 / 0.34 / 0.35).
 void exm_gather_plan(const exm_ctx *ctx, const ChunkInfo &ci, int rc, int *wb_out, int *ng_out)
 {
     int maxn = 0;
@@ -918,7 +919,7 @@ void exm_gather_plan(const exm_ctx *ctx, const ChunkInfo &ci, int rc, int *wb_ou
     wb = std::min(wb, std::max(EXM_WB_MIN, (ctx->nb + 7) / 8 * 8));
     *wb_out = std::max(EXM_WB_MIN, std::min(wb, EXM_WB_MAX));
     const double taps = (double)std::min(tch, std::max(maxn, 1)) * ci.nwalk / EXM_NPAIR;   // of a pair of a block
-    *ng_out = taps >= 12288 ? 4 : (taps >= 3584 ? 2 : 1);
+    *ng_out = taps >= 8000 ? 4 : (taps >= 2500 ? 2 : 1);
 }
 
 // Parts of the 48 plane pairs a (node, lag, template chunk) is split into, each a block of its own: one, or

@@ -8,11 +8,14 @@
 
 #include "common.cuh"
 
-// staging window of one (node, lag, phase plane): rows of beta x columns of Delta.  The row pitch is a
-// multiple of the 32 banks, so the bank of a value depends on its column alone.  The rows are chosen per launch
+// staging window of one (node, lag, phase plane): rows of beta x columns of Delta.  float32: the row pitch is a
+// multiple of the 32 banks, so the bank of a value depends on its column alone, whatever a node's carry.  16 bits: two
+// columns share a bank, and the columns of the taps (a spread of about 14) would crowd a third of the banks; a pitch
+// of 88 words moves each row by 24 banks (a node's carry of one row then changes which taps conflict, which costs less:
+// 1024 templates x 53 nodes x 16 s segments 39.5 ms at 192 columns, NEW16 at 176).  The rows are chosen per launch
 // (exm_gather_plan).
 #define EXM_WD 160     // float32 tables
-#define EXM_WD16 192   // 16-bit tables
+#define EXM_WD16 176   // 16-bit tables
 #define EXM_WB_MIN 80
 #define EXM_WB_MAX 160
 

@@ -334,10 +334,11 @@ __global__ void __launch_bounds__(256) k_tap_scatter(TapArgs a)
 // proposes a bank not yet used, the first of its candidates' from a start that differs from lane to lane and
 // turns with the step; the lowest lane of a bank wins, the others propose again (kOrderRounds1 times; then
 // kOrderRounds2 times for a second tap per bank, then whatever is left).  The fullest bank holds about 26 of
-// a chunk's 512 taps, so 1.6 taps per step is the least any order could reach; this one reaches 2.8 (2.7 with
-// twice the rounds and the fullest banks first), the sorted order 3.6.  One warp per chunk; the banks of a lane's
-// taps are bytes of four registers and the candidates are bit masks.
-constexpr int kOrderRounds1 = 2, kOrderRounds2 = 2;
+// a chunk's 512 taps, so 1.6 taps per step is the least any order could reach; this one reaches 2.9 (2.7 with
+// eight rounds and the fullest banks first), the sorted order 3.6.  More rounds cost this kernel what they save the
+// gather (rounds 1 + 2: gather 63.0 and tap build 10.2 ms, 2 + 2: 62.7 and 10.7, 4 + 3: 62.9 and 11.3).  One warp per chunk;
+// the banks of a lane's taps are bytes of four registers and the candidates are bit masks.
+constexpr int kOrderRounds1 = 1, kOrderRounds2 = 2;
 constexpr int kOrderWarps = 4;
 constexpr int kOrderRow = EXM_GT * EXM_NG_MAX + 1;   // a lane's taps in shared memory, padded against conflicts
 
