@@ -14,13 +14,13 @@
 // path that reads the table from global memory.
 //
 // What bounds it (2048 templates x 53 nodes x 87 lags x 2048 times, 1.65e10 taps): shared-memory reads (eight a
-// tap, 69 % of the data pipe) and instruction issue (61 %) together; DRAM is at a tenth of its rate.  92.7 -> 62.7 ms:
+// tap, 79 % of the data pipe) and instruction issue (63 %) together; DRAM is at a tenth of its rate.  92.7 -> 61.3 ms:
 //  * four taps of one template per group: the bookkeeping of templates, the ranges and the running maximum are paid
 //    once for four taps (5.4 -> 2.8 warp instructions per tap); padding the runs to whole groups adds 3.8 % taps;
 //  * a row pitch of a multiple of the 32 banks, and taps ordered so that a step's lanes hit different banks
-//    (k_tap_order): 3.4 -> 2.4 cycles per read;
+//    (k_tap_order): 3.4 -> 2.5 cycles per read;
 //  * boundary points in blocks of their own, so the accumulators take 24 instead of 80 bytes a template and a block
-//    takes 1024 templates: every plane pair costs a block a fixed ~6 us of waits (68.0 at 704, 75.5 at 352);
+//    takes up to 2048 templates: every plane pair costs a block a fixed ~1.7 us of waits (planes_tch);
 //  * a warp's first descriptors and end templates of the next pair loaded before it waits for that pair's planes.
 //  * descriptors loaded by whole chunks: no lane's loads are predicated or replaced by constants (65.3 -> 62.7).
 // 20 warps at 96 registers: 16 warps 64.2 ms (too few to cover the latencies), 24 and 28 spill (68.4, 80).
@@ -560,9 +560,10 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar)
 // EXM_SLOWQ int2 entries (storage index of the tap; template | random flag << 29)
 #define EXM_ACC_F 6    // floats per template: three sets of (m, S)
 #define EXM_ACCB_F 8   // ... of a boundary block: and bcf, bsh
-#define EXM_EDGE_B (4 * 2 * EXM_EDGE_F * 32)
+#define EXM_MAX_NC 27  // most consumer warps of a launch shape
+#define EXM_EDGE_B (4 * 2 * EXM_EDGE_F * EXM_MAX_NC)
 #define EXM_QCNT_B (4 * 3 * 32)
-#define EXM_QENT_B (8 * 3 * 32 * EXM_SLOWQ)
+#define EXM_QENT_B (8 * 3 * EXM_MAX_NC * EXM_SLOWQ)
 #define EXM_GATHER_FIXED_B (64 + EXM_EDGE_B + EXM_QCNT_B + EXM_QENT_B)
 
 // Warp NW - 1 is the producer: it stages the planes with TMA and, once every consumer warp has
@@ -577,6 +578,7 @@ __global__ void __launch_bounds__(NW * 32, 1) k_gather_planes(const __grid_const
                                                                 const __grid_constant__ PlaneArgs a)
 {
     constexpr int NC = NW - 1;   // consumer warps
+    static_assert(NC <= EXM_MAX_NC, "shared memory is laid out for EXM_MAX_NC consumers");
     const int SLOT = a.wb * TabElem<TE>::wd;
     const unsigned SLOT_B = (unsigned)SLOT * (unsigned)sizeof(TE);
     unsigned char *smem = exm_gsm;
@@ -699,7 +701,7 @@ __global__ void __launch_bounds__(NW * 32, 1) k_gather_planes(const __grid_const
                     }
                     const int wexcl = __shfl_sync(0xffffffffu, excl, wi);
                     if (i < total) {
-                        const int2 e = qent[(par * 32 + wi) * EXM_SLOWQ + (i - wexcl)];
+                        const int2 e = qent[(par * NC + wi) * EXM_SLOWQ + (i - wexcl)];
                         const int il = e.y & 0x1FFF;
                         const int tm = tsr_all[e.x];
                         v = bnd ? slow_tap<true, TE>(a, il, tm, k, r, a.m_base, a.tsc[k])
@@ -776,7 +778,7 @@ __global__ void __launch_bounds__(NW * 32, 1) k_gather_planes(const __grid_const
             if (lane == 0) qcnt[(p % 3) * 32 + warp] = 0;
             __syncwarp();
             rc.qn = qcnt_o + 4u * ((p % 3) * 32 + warp);
-            rc.q = qent_o + 8u * (((p % 3) * 32 + warp) * EXM_SLOWQ);
+            rc.q = qent_o + 8u * (((p % 3) * NC + warp) * EXM_SLOWQ);
             if (!ok) {   // no work: empty edge slots for the producer
                 rc.tF = rc.tL = -1;
                 rc.beg = rc.end = 0;
@@ -886,7 +888,8 @@ static int planes_tch_max(const exm_ctx *ctx, int wb)
 
 // templates per gather block: pct / 150 of the most that still gives every SM eight blocks (a block's start,
 // the waits at each plane pair and the staging of its windows are paid once for all its templates), between
-// 256 and EXM_TCH_PLAN at 150
+// 256 and EXM_TCH_PLAN at 150, then the same for every chunk of a node.  2048 templates x 53 nodes at 352 / 512 / 704 /
+// 1024 / 2048: 75.5 / 70.9 / 68.0 / 65.4 ms, and on a later kernel 65.2 / 63.1 / 61.1 at the last three.
 static int planes_tch(const exm_ctx *ctx, const ChunkInfo &ci, int rc, int pct, int *maxn_out)
 {
     long long pairs = 0;
@@ -901,7 +904,8 @@ static int planes_tch(const exm_ctx *ctx, const ChunkInfo &ci, int rc, int pct, 
     tch = std::min<long long>(std::max<long long>(tch, 256), EXM_TCH_PLAN);
     tch = std::min<long long>(tch * pct / 150, EXM_TCH);
     tch = std::max<long long>(1, std::min<long long>(tch, maxn));
-    return (int)((tch + 15) / 16 * 16);
+    const long long nch = std::max<long long>(1, (maxn + tch - 1) / tch);
+    return (int)(((maxn + nch - 1) / nch + 15) / 16 * 16);
 }
 
 // The windows' height and the descriptors' chunk, which the tap build and the gather share.  Rows: the most that
@@ -912,7 +916,7 @@ static int planes_tch(const exm_ctx *ctx, const ChunkInfo &ci, int rc, int pct, 
 void exm_gather_plan(const exm_ctx *ctx, const ChunkInfo &ci, int rc, int *wb_out, int *ng_out)
 {
     int maxn = 0;
-    const int tch = planes_tch(ctx, ci, rc, 150, &maxn);
+    const int tch = std::max(16, planes_tch(ctx, ci, rc, 150, &maxn));
     const size_t fixed = EXM_GATHER_FIXED_B + 2048 + (size_t)tch * EXM_ACC_F * 4;
     const size_t row = 3 * (size_t)exm_dtype_wd(ctx->dtype) * exm_dtype_bytes(ctx->dtype);
     int wb = (int)((ctx->smem_optin - fixed) / row) / 8 * 8;
@@ -929,7 +933,7 @@ int exm_gather_parts(const exm_ctx *ctx, int nmc, int m_base, int nwalk, int rc)
     (void)nwalk;
     int maxn = 0;
     ChunkInfo ci{m_base, nmc, nwalk, 0, 0.f};
-    const int tch = planes_tch(ctx, ci, rc, 150, &maxn);
+    const int tch = std::max(16, planes_tch(ctx, ci, rc, 150, &maxn));
     const long long blocks = (long long)rc * ctx->nn * ((maxn + tch - 1) / std::max(tch, 1));
     const long long waves = blocks / std::max(1, ctx->sm_count);
     return waves >= 8 ? 1 : (waves >= 4 ? 2 : 4);

@@ -12,7 +12,7 @@
 // multiple of the 32 banks, so the bank of a value depends on its column alone, whatever a node's carry.  16 bits: two
 // columns share a bank, and the columns of the taps (a spread of about 14) would crowd a third of the banks; a pitch
 // of 88 words moves each row by 24 banks (a node's carry of one row then changes which taps conflict, which costs less:
-// 1024 templates x 53 nodes x 16 s segments 39.5 ms at 192 columns, NEW16 at 176).  The rows are chosen per launch
+// 1024 templates x 53 nodes x 16 s segments 39.5 ms at 192 columns, 34.9 at 176).  The rows are chosen per launch
 // (exm_gather_plan).
 #define EXM_WD 160     // float32 tables
 #define EXM_WD16 176   // 16-bit tables
@@ -49,7 +49,7 @@ inline size_t exm_dtype_bytes(int dtype) { return dtype == EXM_DTYPE_F32 ? 4 : 2
 inline int exm_dtype_wd(int dtype) { return dtype == EXM_DTYPE_F32 ? EXM_WD : EXM_WD16; }
 inline int exm_dtype_calign(int dtype) { return dtype == EXM_DTYPE_F32 ? 4 : 8; }
 #define EXM_TCH 2048        // templates per gather block
-#define EXM_TCH_PLAN 1024   // ... by default
+#define EXM_TCH_PLAN 2048   // ... by default
 
 // Tap descriptors of one lag are sorted by (plane pair, template) and each (pair, template) run is padded to
 // whole groups of EXM_GT taps, so that every group has one template.  They are stored in chunks of 32 EXM_GT ng
