@@ -340,13 +340,10 @@ __global__ void __launch_bounds__(256) k_tap_scatter(TapArgs a)
 // the banks of a lane's taps are bytes of four registers and the candidates are bit masks.
 constexpr int kOrderRounds1 = 1, kOrderRounds2 = 2;
 constexpr int kOrderWarps = 4;
-constexpr int kOrderRow = EXM_GT * EXM_NG_MAX + 1;   // a lane's taps in shared memory, padded against conflicts
-
-struct OrderSmem {
-    uint4 d[32 * kOrderRow];
-    int32_t t[32 * kOrderRow];
-    unsigned claim[32];   // per bank: the round's number << 5 | 31 - lane of its lowest proposer
-};
+// a warp's shared memory: the chunk, a lane's taps padded by one against conflicts, and per bank the claim of a
+// round (its number << 5 | 31 - lane of the lowest proposer).  It is as small as the chunk: the kernel waits on
+// its own short chains, and small chunks leave room for more warps.
+inline size_t order_warp_bytes(int ng) { return (32 * (EXM_GT * ng + 1)) * (sizeof(uint4) + sizeof(int32_t)) + 32 * sizeof(unsigned); }
 
 __global__ void __launch_bounds__(32 * kOrderWarps) k_tap_order(uint4 *__restrict__ desc, int32_t *__restrict__ tside,
                                                                 const int *__restrict__ cnt, int nmc, long long pitch,
@@ -356,13 +353,15 @@ __global__ void __launch_bounds__(32 * kOrderWarps) k_tap_order(uint4 *__restric
     extern __shared__ unsigned char osm[];
     __shared__ int pair0[EXM_NPAIR];   // the first position of each plane pair
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    OrderSmem &sm = ((OrderSmem *)osm)[warp];
-    const int rl = blockIdx.y, tpl = EXM_GT * ng, size = 32 * tpl;
+    const int rl = blockIdx.y, tpl = EXM_GT * ng, size = 32 * tpl, row_d = tpl + 1;
+    uint4 *sm_d = (uint4 *)(osm + (size_t)warp * (32 * row_d * (sizeof(uint4) + sizeof(int32_t)) + 32 * sizeof(unsigned)));
+    int32_t *sm_t = (int32_t *)(sm_d + 32 * row_d);
+    unsigned *sm_claim = (unsigned *)(sm_t + 32 * row_d);
     if (threadIdx.x < EXM_NPAIR) pair0[threadIdx.x] = cnt[((long long)rl * EXM_NPAIR + threadIdx.x) * (nmc + 1)];
     __syncthreads();
     const int used_taps = (int)min((long long)cnt[(long long)(rl + 1) * EXM_NPAIR * (nmc + 1) - 1], pitch);
     const int n_chunks = (used_taps + size - 1) / size;
-    sm.claim[lane] = 0u;
+    sm_claim[lane] = 0u;
     unsigned stamp = 0u;
     for (int ch = blockIdx.x * kOrderWarps + warp; ch < n_chunks; ch += gridDim.x * kOrderWarps) {
         uint4 *d = desc + rl * pitch + (long long)ch * size;
@@ -371,13 +370,13 @@ __global__ void __launch_bounds__(32 * kOrderWarps) k_tap_order(uint4 *__restric
         for (int q = lane; q < size; q += 32) {
             const bool in = ch * size + q < used_taps;
             const uint4 v = in ? d[q] : make_uint4(0u, 0u, 0u, EXM_DESC_PAD);
-            const int at = (q / tpl) * kOrderRow + q % tpl;
-            sm.d[at] = v;
-            sm.t[at] = in ? t[q] : 0;
+            const int at = (q / tpl) * row_d + q % tpl;
+            sm_d[at] = v;
+            sm_t[at] = in ? t[q] : 0;
         }
         __syncwarp();
         // this lane's taps: their banks, and per group the lane's groups of the same run
-        const uint4 *row = sm.d + lane * kOrderRow;
+        const uint4 *row = sm_d + lane * row_d;
         unsigned bk[EXM_NG_MAX], same[EXM_NG_MAX], tm[EXM_NG_MAX];
 #pragma unroll
         for (int g = 0; g < EXM_NG_MAX; ++g) {
@@ -438,9 +437,9 @@ __global__ void __launch_bounds__(32 * kOrderWarps) k_tap_order(uint4 *__restric
                         taken |= asked;
                         // the lowest lane that proposes the same bank
                         stamp += 32u;
-                        if (av) atomicMax(&sm.claim[r], stamp | (31u - lane));
+                        if (av) atomicMax(&sm_claim[r], stamp | (31u - lane));
                         __syncwarp();
-                        if (av && sm.claim[r] == (stamp | (31u - lane))) pick = r;
+                        if (av && sm_claim[r] == (stamp | (31u - lane))) pick = r;
                         __syncwarp();
                     }
                 }
@@ -455,9 +454,9 @@ __global__ void __launch_bounds__(32 * kOrderWarps) k_tap_order(uint4 *__restric
                 if ((eq & (eq - 1u)) == 0u) banks &= ~(1u << pick);
                 cand &= ~(1u << j);
                 rem &= ~(1u << j);
-                const int at = lane * kOrderRow + j, ph = (g * EXM_GT + u) * 32 + lane;
-                d[ph] = sm.d[at];
-                t[ph] = sm.t[at];
+                const int at = lane * row_d + j, ph = (g * EXM_GT + u) * 32 + lane;
+                d[ph] = sm_d[at];
+                t[ph] = sm_t[at];
             }
         }
         __syncwarp();
@@ -526,12 +525,13 @@ __global__ void __launch_bounds__(1024) k_windows(const int *hist_b, const int *
     if (tid < nn) win[1 + tid] = max(0, min(rh + cki[tid], nb - wb));
 }
 
-// Parts of the walked times in the count: as many as give each SM about 32 warps of lags, of at least 64 times
+// Parts of the walked times in the count: as many as give each SM about 16 warps of lags, of at least 64 times (more
+// parts cost more than they bring: every part writes its own counts, each to a sector of its own)
 int exm_tap_parts(const exm_ctx *ctx, int nmc, int nwalk, int rc)
 {
     const long long warps = (long long)nmc * ((rc + 31) / 32);
     long long nq = 1;
-    while (nq < 32 && warps * nq < 32LL * ctx->sm_count && nwalk / (2 * nq) >= 64) nq *= 2;
+    while (nq < 32 && warps * nq < 16LL * ctx->sm_count && nwalk / (2 * nq) >= 64) nq *= 2;
     return (int)nq;
 }
 
@@ -582,10 +582,10 @@ void exm_run_taps(exm_ctx *ctx, exm_slot &sl, const ChunkInfo &ci, int r0, int r
     const int lag_parts = std::min(rc, std::max(1, (12 * ctx->sm_count + ci.nmc - 1) / ci.nmc));
     k_tap_scatter<<<dim3(ci.nmc, lag_parts), 256, std::min(kScatterCache, ci.nwalk) * sizeof(WalkEntry), ctx->stream>>>(a);
     const long long n_chunks = a.pitch / (32 * EXM_GT * sl.ng);
-    const size_t osm = kOrderWarps * sizeof(OrderSmem);
+    const size_t osm = kOrderWarps * order_warp_bytes(sl.ng);
     exm_allow_smem(ctx, (const void *)k_tap_order, osm);
     const dim3 go((unsigned)std::min<long long>((n_chunks + kOrderWarps - 1) / kOrderWarps,
-                                                std::max(1, ctx->sm_count * 20 / rc)), rc);
+                                                std::max(1, ctx->sm_count * 40 / rc)), rc);
     k_tap_order<<<go, 32 * kOrderWarps, osm, ctx->stream>>>(a.desc, a.tside, a.cnt, ci.nmc, a.pitch, sl.ng,
                                                            ctx->dtype == EXM_DTYPE_F32 ? 0 : 1);
     EXM_CUDA(cudaGetLastError());
