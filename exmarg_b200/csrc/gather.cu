@@ -927,16 +927,17 @@ void exm_gather_plan(const exm_ctx *ctx, const ChunkInfo &ci, int rc, int *wb_ou
 }
 
 // Parts of the 48 plane pairs a (node, lag, template chunk) is split into, each a block of its own: one, or
-// more when the launch has too few blocks to keep the SMs busy to the end.
+// more when the launch has too few blocks to keep the SMs busy to the end.  Gather ms at 1 / 2 / 4 / 8 parts:
+// 3.5 waves of blocks (24 templates, every time) 1.22 / 1.05 / 0.97 / 1.00, (150 x 6 nodes) 1.66 / 1.49 / 1.45 / 1.50; 9.5
+// waves (333 x 21, two segments) 6.81 / 6.58 / 6.67 / 6.96; 15 waves (58 x 53) 1.92 / 1.93 / 2.04 / 2.28.
 int exm_gather_parts(const exm_ctx *ctx, int nmc, int m_base, int nwalk, int rc)
 {
-    (void)nwalk;
     int maxn = 0;
-    ChunkInfo ci{m_base, nmc, nwalk, 0, 0.f};
+    const ChunkInfo ci{m_base, nmc, nwalk, 0, 0.f};
     const int tch = std::max(16, planes_tch(ctx, ci, rc, 150, &maxn));
     const long long blocks = (long long)rc * ctx->nn * ((maxn + tch - 1) / std::max(tch, 1));
     const long long waves = blocks / std::max(1, ctx->sm_count);
-    return waves >= 8 ? 1 : (waves >= 4 ? 2 : 4);
+    return waves >= 12 ? 1 : (waves >= 4 ? 2 : 4);
 }
 
 void exm_run_gather_planes(exm_ctx *ctx, exm_slot &sl, const ChunkInfo &ci, int r0, int rc)
