@@ -93,26 +93,30 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem, bool va
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(gmem), "r"(valid ? 16 : 0));
 }
 
-// RG row groups of 8 nodes and QG = 8 / RG groups of threads that share out the quadrature points: thread
-// (tc, rg, qg) holds 8 nodes x 8 keys (x0 + c, y0 + tc) over the points qg, qg + QG, ... of each step, and the
-// point groups' sums are added at the end.  Bound by the float64 pipe: the fewest rows that hold the nodes cost
-// the fewest operations.  Per pixel at order 120: 6 nodes 12.1 ms, 14 nodes 20.5, 30 nodes 38.1, 53 nodes 67.2; one tile
-// of 64 rows with its products staged in shared memory (three barriers a step) took 79 ms whatever the nodes.
-constexpr int w_rows(int rg) { return 8 * rg + kWX + kWY + 1; }
-constexpr size_t w_smem(int rg)
+// RG row groups of R nodes and QG = 8 / RG groups of threads that share out the quadrature points: thread
+// (tc, rg, qg) holds R nodes x 8 keys (x0 + c, y0 + tc) over the points qg, qg + QG, ... of each step, and the
+// point groups' sums are added at the end.  Bound by the float64 pipe and its latency: the fewest rows that hold the
+// nodes cost the fewest operations, and fewer sums a thread leave registers for three or four blocks an SM (R <= 7,
+// R <= 4) instead of two.  Per pixel at order 120: 6 nodes 8.9 ms, 14 nodes 17.4, 30 nodes 38.1, 53 nodes 55.9; groups
+// of 8 rows whatever the nodes took 12.1, 20.4, 38.1, 67.2, and one tile of 64 rows with its products staged in shared
+// memory (three barriers a step) 79.  Twice the row groups of half the rows were slower (6 nodes 10.0, 14 nodes 21.4)
+// but at exactly 8 nodes (11.9 against 12.2): each thread forms the products of its keys again for fewer rows.
+constexpr int w_rows(int rg, int r) { return r * rg + kWX + kWY + 1; }
+constexpr int w_blocks(int r) { return r <= 4 ? 4 : r <= 7 ? 3 : 2; }
+constexpr size_t w_smem(int rg, int r)
 {
-    const size_t st = sizeof(double) * kWStages * w_rows(rg) * kWPitch;
+    const size_t st = sizeof(double) * kWStages * w_rows(rg, r) * kWPitch;
     return st > 32768 ? st : 32768;   // at the end: 32 KB of sums to add
 }
 
-template <int RG>
-__global__ void __launch_bounds__(kWThreads, 2) k_w_gemm(const int4 *__restrict__ tiles, int Qp, int n_nodes, int n_max,
+template <int RG, int R>
+__global__ void __launch_bounds__(kWThreads, w_blocks(R)) k_w_gemm(const int4 *__restrict__ tiles, int Qp, int n_nodes, int n_max,
                                                          const double *__restrict__ lad1, const double *__restrict__ lad2,
                                                          const double *__restrict__ cm, const double *__restrict__ bw,
                                                          int t0, double w0, double w1, int n_tau, long long n_keys,
                                                          double *__restrict__ Wraw)
 {
-    constexpr int QG = 8 / RG, NR = w_rows(RG);
+    constexpr int QG = 8 / RG, NR = w_rows(RG, R);
     extern __shared__ __align__(16) double wsm[];   // [stage][row: nodes, x ladder, y ladder, cos][point]
     const int4 tl = tiles[blockIdx.x];
     const int m = tl.x, x0 = tl.y, y0 = tl.z;
@@ -125,15 +129,15 @@ __global__ void __launch_bounds__(kWThreads, 2) k_w_gemm(const int4 *__restrict_
             const int row = i / (kWQ / 2), qq = 2 * (i - row * (kWQ / 2));
             const double *src = bw;
             bool ok;
-            if (row < 8 * RG) {
+            if (row < R * RG) {
                 ok = row < n_nodes;
                 if (ok) src = bw + (size_t)row * Qp;
-            } else if (row < 8 * RG + kWX) {
-                const int x = x0 + row - 8 * RG;
+            } else if (row < R * RG + kWX) {
+                const int x = x0 + row - R * RG;
                 ok = x <= L - 1;
                 if (ok) src = lad1 + (size_t)(m + 2 * x) * Qp;
-            } else if (row < 8 * RG + kWX + kWY) {
-                const int y = y0 + row - 8 * RG - kWX;
+            } else if (row < R * RG + kWX + kWY) {
+                const int y = y0 + row - R * RG - kWX;
                 ok = y <= L - 1;
                 if (ok) src = lad2 + (size_t)(m + 2 * y) * Qp;
             } else {
@@ -143,9 +147,9 @@ __global__ void __launch_bounds__(kWThreads, 2) k_w_gemm(const int4 *__restrict_
             cp_async16(st + row * kWPitch + qq, src + (ok ? step * kWQ + qq : 0), ok);
         }
     };
-    double acc[8][8];
+    double acc[R][8];
 #pragma unroll
-    for (int r = 0; r < 8; ++r)
+    for (int r = 0; r < R; ++r)
 #pragma unroll
         for (int c = 0; c < 8; ++c) acc[r][c] = 0.0;
 #pragma unroll
@@ -159,18 +163,18 @@ __global__ void __launch_bounds__(kWThreads, 2) k_w_gemm(const int4 *__restrict_
         if (k + kWStages - 1 < nsteps) issue(k + kWStages - 1, (k + kWStages - 1) % kWStages);
         asm volatile("cp.async.commit_group;\n" ::);
         const double *st = wsm + (size_t)(k % kWStages) * NR * kWPitch;
-        const double *pa = st + rg * 8 * kWPitch, *px = st + 8 * RG * kWPitch;
-        const double *py = st + (8 * RG + kWX + tc) * kWPitch, *pc = st + (8 * RG + kWX + kWY) * kWPitch;
+        const double *pa = st + rg * R * kWPitch, *px = st + R * RG * kWPitch;
+        const double *py = st + (R * RG + kWX + tc) * kWPitch, *pc = st + (R * RG + kWX + kWY) * kWPitch;
 #pragma unroll 2
         for (int qq = qg; qq < kWQ; qq += QG) {
             const double yc = __dmul_rn(py[qq], pc[qq]);
-            double a[8], b[8];
+            double a[R], b[8];
 #pragma unroll
-            for (int r = 0; r < 8; ++r) a[r] = pa[r * kWPitch + qq];
+            for (int r = 0; r < R; ++r) a[r] = pa[r * kWPitch + qq];
 #pragma unroll
             for (int c = 0; c < 8; ++c) b[c] = __dmul_rn(px[c * kWPitch + qq], yc);
 #pragma unroll
-            for (int r = 0; r < 8; ++r)
+            for (int r = 0; r < R; ++r)
 #pragma unroll
                 for (int c = 0; c < 8; ++c) acc[r][c] = fma(a[r], b[c], acc[r][c]);
         }
@@ -180,23 +184,23 @@ __global__ void __launch_bounds__(kWThreads, 2) k_w_gemm(const int4 *__restrict_
 #pragma unroll
     for (int h = QG / 2; h > 0; h /= 2) {
         __syncthreads();
-        double *red = wsm + (size_t)((qg % h) * RG + rg) * 64 * 16 + tc;
+        double *red = wsm + (size_t)((qg % h) * RG + rg) * R * 8 * 16 + tc;
         if (qg >= h && qg < 2 * h)
 #pragma unroll
-            for (int r = 0; r < 8; ++r)
+            for (int r = 0; r < R; ++r)
 #pragma unroll
                 for (int c = 0; c < 8; ++c) red[(r * 8 + c) * 16] = acc[r][c];
         __syncthreads();
         if (qg < h)
 #pragma unroll
-            for (int r = 0; r < 8; ++r)
+            for (int r = 0; r < R; ++r)
 #pragma unroll
                 for (int c = 0; c < 8; ++c) acc[r][c] = __dadd_rn(acc[r][c], red[(r * 8 + c) * 16]);
     }
     if (qg) return;
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        const int row = rg * 8 + r;
+    for (int r = 0; r < R; ++r) {
+        const int row = rg * R + r;
         if (row >= n_nodes) continue;
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
@@ -289,10 +293,10 @@ extern "C" int exm_w_build(exm_ctx *ctx, int n_nodes, const double *s_nodes, int
         EXM_CUDA(cudaEventCreate(&e1));
         EXM_CUDA(cudaEventCreate(&e2));
         EXM_CUDA(cudaEventRecord(e0, ctx->stream));
-        auto gemm = [&](auto rg, int p) {
-            constexpr int RG = decltype(rg)::value;
-            exm_allow_smem(ctx, (const void *)k_w_gemm<RG>, w_smem(RG));
-            k_w_gemm<RG><<<(int)tiles.size(), kWThreads, w_smem(RG), ctx->stream>>>(
+        auto gemm = [&](auto rg, auto rr, int p) {
+            constexpr int RG = decltype(rg)::value, R = decltype(rr)::value;
+            exm_allow_smem(ctx, (const void *)k_w_gemm<RG, R>, w_smem(RG, R));
+            k_w_gemm<RG, R><<<(int)tiles.size(), kWThreads, w_smem(RG, R), ctx->stream>>>(
                 (const int4 *)d_tiles.p, Qp, n_nodes, n_max, (const double *)d_l1.p, (const double *)d_l2.p,
                 (const double *)d_cm.p, (const double *)d_bw.p, j0[p], w[2 * p], w[2 * p + 1], n_tau, n_keys,
                 (double *)d_W.p);
@@ -306,15 +310,26 @@ extern "C" int exm_w_build(exm_ctx *ctx, int n_nodes, const double *s_nodes, int
                                                                 (double *)d_l2.p, (double *)d_dph.p, (double *)d_bw.p);
             k_w_cos<<<dim3((Qp + 127) / 128, n_max + 1), 128, 0, ctx->stream>>>((const double *)d_dph.p, Qp,
                                                                                (double *)d_cm.p);
-            // the fewest rows that hold the nodes
-            if (n_nodes <= 8)
-                gemm(std::integral_constant<int, 1>(), p);
-            else if (n_nodes <= 16)
-                gemm(std::integral_constant<int, 2>(), p);
-            else if (n_nodes <= 32)
-                gemm(std::integral_constant<int, 4>(), p);
-            else
-                gemm(std::integral_constant<int, 8>(), p);
+            // the fewest rows that hold the nodes: one row group up to 8 nodes, else 5 to 8 rows in each of 2, 4 or 8
+            const int rg = n_nodes <= 8 ? 1 : n_nodes <= 16 ? 2 : n_nodes <= 32 ? 4 : 8;
+            auto rows = [&](auto r) {
+                if (rg == 1) gemm(std::integral_constant<int, 1>(), r, p);
+                if constexpr (decltype(r)::value >= 5) {
+                    if (rg == 2) gemm(std::integral_constant<int, 2>(), r, p);
+                    if (rg == 4) gemm(std::integral_constant<int, 4>(), r, p);
+                    if (rg == 8) gemm(std::integral_constant<int, 8>(), r, p);
+                }
+            };
+            switch ((n_nodes + rg - 1) / rg) {
+                case 1: rows(std::integral_constant<int, 1>()); break;
+                case 2: rows(std::integral_constant<int, 2>()); break;
+                case 3: rows(std::integral_constant<int, 3>()); break;
+                case 4: rows(std::integral_constant<int, 4>()); break;
+                case 5: rows(std::integral_constant<int, 5>()); break;
+                case 6: rows(std::integral_constant<int, 6>()); break;
+                case 7: rows(std::integral_constant<int, 7>()); break;
+                default: rows(std::integral_constant<int, 8>()); break;
+            }
         }
         EXM_CUDA(cudaGetLastError());
         EXM_CUDA(cudaEventRecord(e1, ctx->stream));
