@@ -12,6 +12,7 @@ tables stay resident and the device path sizes its own launches.  With a 'cpu' o
 
 import json
 import os
+import zlib
 
 import numpy as np
 
@@ -107,11 +108,12 @@ def tune_cache_path():
 
 
 def tune_key(ctx, n_loud, n_random):
-    """the workload shape the gather's best launch depends on, and the device model (its memory size)"""
+    """the workload shape the gather's best launch depends on, the device model (its memory size) and the
+    list of launch shapes (an entry is an index into it: one recorded with another list is not taken)"""
     nn, ntau, nphif, nb, nd, dtype = ctx.store_shape
-    return "dev%d|templates%d|n_time%d|nodes%d|lags%d|planes%d|nb%d|nd%d|dtype%d|walk%d" % (
+    return "dev%d|templates%d|n_time%d|nodes%d|lags%d|planes%d|nb%d|nd%d|dtype%d|walk%d|shapes%08x" % (
         int(ctx.device_total) >> 30, ctx.nm, ctx.n_time, nn, ntau, nphif, nb, nd, dtype,
-        (n_loud + n_random) if n_loud > 0 else ctx.n_time)
+        (n_loud + n_random) if n_loud > 0 else ctx.n_time, zlib.crc32(",".join(_lib.GATHER_SHAPES).encode()))
 
 
 def _read_cache(path):
