@@ -158,9 +158,9 @@ def measured_peaks():
 # read per node-tap both do), so the full launch's traffic is this figure times its node-taps.  The capture
 # holds only for the kernel sources it was taken on: if they changed since, traffic is reported as null.
 GATHER_TRAFFIC = {
-    "dram_bytes_per_node_tap": 3.9683,       # (1.8772e9 + 8.92e6) B / 4.7531e8 node-taps (28 warps x 1, 150 %)
-    "l2_read_hit_rate": 69.92,             # lts__t_sector_op_read_hit_rate.pct
-    "sources_sha256": "6014a92f6f6972047daeb8f5535a10d004f69fd2b89c0258d722db9f213bc2f9",
+    "dram_bytes_per_node_tap": 8.6897,       # (4.1217e9 + 8.65e6) B / 4.7531e8 node-taps (20 warps x 2)
+    "l2_read_hit_rate": 64.13,             # lts__t_sector_op_read_hit_rate.pct
+    "sources_sha256": "343507eb60a2d3ab1b2f0cc1fa4558a68bdf37713239eed51cb51f48181ab392",
     "capture": "profiles/k_gather_planes_small.md",
 }
 GATHER_SOURCES = ("exmarg_b200/csrc/gather.cu", "exmarg_b200/csrc/taps.cu", "exmarg_b200/csrc/kernels.cuh")
@@ -666,7 +666,8 @@ def w_build_leg(args, local):
         L = wtable.N_MAX - m + 1
         for x0 in range(0, L, 8):
             tiles += len(range(0, L - x0, 16))
-    exec_tf = 2.0 * tiles * 64 * 128 * q / (per_px * 1e-3) / 1e12
+    groups = next(g for g in (1, 2, 4, 8) if s_nodes.size <= 8 * g)      # row groups of the fewest rows that hold the nodes
+    exec_tf = 2.0 * tiles * (-(-int(s_nodes.size) // groups) * groups) * 128 * q / (per_px * 1e-3) / 1e12
     out = {"pixels_run": int(pix.size), "ms_per_pixel": per_px, "projected_build_s": per_px * 1e-3 * npix,
            "reference_published_s": 7.1 * 3600, "reference_published": "7.1 h for the 53 nodes on one GPU (build_w.py:5-6)",
            "nodes": int(s_nodes.size), "fp64_fma_per_pixel": fma, "fp64_tflops_useful": 2 * fma / (per_px * 1e-3) / 1e12,

@@ -163,7 +163,7 @@ class Context:
         self.prep_token = None
         self.nm = self.nfreq = self.n_time = None
         self.gather_cfg = None          # the launch shape chosen by autotune or set_gather_cfg (None: default)
-        self.gather_chunk_pct = 150     # templates per gather block, percent of one wave of blocks per lag
+        self.gather_chunk_pct = 150     # templates per gather block (150: the library's own choice)
         self.store_shape = None         # (nodes, lags, phase planes, nb, nd, dtype) of the resident store
         self.device_total = device_memory(device)[1]   # identifies the device model in the autotune cache
 
