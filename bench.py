@@ -160,7 +160,7 @@ def measured_peaks():
 GATHER_TRAFFIC = {
     "dram_bytes_per_node_tap": 8.6897,       # (4.1217e9 + 8.65e6) B / 4.7531e8 node-taps (20 warps x 2)
     "l2_read_hit_rate": 64.13,             # lts__t_sector_op_read_hit_rate.pct
-    "sources_sha256": "343507eb60a2d3ab1b2f0cc1fa4558a68bdf37713239eed51cb51f48181ab392",
+    "sources_sha256": "e3ad869d64ebbd1aaf4fec5c123e9433565c1b6a64cb17609788c3620331658d",
     "capture": "profiles/k_gather_planes_small.md",
 }
 GATHER_SOURCES = ("exmarg_b200/csrc/gather.cu", "exmarg_b200/csrc/taps.cu", "exmarg_b200/csrc/kernels.cuh")

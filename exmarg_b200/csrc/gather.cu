@@ -2,7 +2,7 @@
 //
 // k_gather_planes (the pe_intrinsic path): one block per (lag r, template chunk, node k).  The block walks
 // the 48 phase-plane pairs (p, p+1) of the node's lag slab T[k, r]; for each plane it stages, with one TMA
-// copy, a window of 80-160 beta rows x 160 (16-bit tables: 192) Delta columns into shared memory (three
+// copy, a window of 80-160 beta rows x 160 (16-bit tables: 176) Delta columns into shared memory (three
 // slots: two planes in use, one in flight).  The descriptors of the lag are sorted by (plane pair,
 // template) in groups of four taps of one template, and each warp owns a contiguous range of groups: it
 // evaluates the bilinear x linear interpolation of a lane's four taps from shared memory, takes their maximum and
