@@ -664,8 +664,12 @@ def w_build_leg(args, local):
     tiles = 0
     for m in range(wtable.N_MAX + 1):
         L = wtable.N_MAX - m + 1
-        for x0 in range(0, L, 8):
-            tiles += len(range(0, L - x0, 16))
+        x0 = y0 = 0
+        while x0 < L:                                # columns of 8 keys, 16 to a tile, one x-block after the other
+            tiles, na = tiles + 1, min(16, L - x0 - y0)
+            x0, y0 = (x0 + 8, 16 - na) if na < 16 else (x0, y0 + 16)
+            if x0 + y0 >= L:
+                x0, y0 = x0 + 8, 0
     groups = next(g for g in (1, 2, 4, 8) if s_nodes.size <= 8 * g)      # row groups of the fewest rows that hold the nodes
     exec_tf = 2.0 * tiles * (-(-int(s_nodes.size) // groups) * groups) * 128 * q / (per_px * 1e-3) / 1e12
     out = {"pixels_run": int(pix.size), "ms_per_pixel": per_px, "projected_build_s": per_px * 1e-3 * npix,

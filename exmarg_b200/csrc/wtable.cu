@@ -12,10 +12,11 @@
 //             power ladders m_I^k (k = 0 .. 2 n_max), dph and the damping Bw_j of every node;
 //   k_w_cos:  cos(m dph_q) of every phase class m;
 //   k_w_gemm: for a phase class m the keys form the triangle pw1 = m + 2x, pw2 = m + 2y, x + y <= n_max - m.
-//             A block takes a tile of 8 x-values by 16 y-values (128 keys) and 8 RG rows (nodes): a
-//             register-tiled float64 product over q, A[j][q] = Bw_j(q) and B[q][(x, y)] = m1_q^pw1 (m2_q^pw2
-//             cos(m dph_q)), formed in registers from the tile's 8 + 16 ladder rows; three stages of inputs
-//             arrive by asynchronous copies, one block barrier a step.
+//             The triangle's columns of 8 x-values (x0 .. x0 + 7, y), y <= n_max - m - x0, are laid out one x-block
+//             after the other, and a block takes 16 of them (128 keys, of one x-block and perhaps the next) and R RG
+//             rows (nodes): a register-tiled float64 product over q, A[j][q] = Bw_j(q) and B[q][(x, y)] = m1_q^pw1
+//             (m2_q^pw2 cos(m dph_q)), formed in registers from the tile's 8 or 16 + 16 ladder rows; three stages of
+//             inputs arrive by asynchronous copies, one block barrier a step.
 //   k_w_scale: W = Wraw * scale, rounded to float32, non-finite entries counted.
 #include <type_traits>
 #include <vector>
@@ -97,11 +98,13 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem, bool va
 // (tc, rg, qg) holds R nodes x 8 keys (x0 + c, y0 + tc) over the points qg, qg + QG, ... of each step, and the
 // point groups' sums are added at the end.  Bound by the float64 pipe and its latency: the fewest rows that hold the
 // nodes cost the fewest operations, and fewer sums a thread leave registers for three or four blocks an SM (R <= 7,
-// R <= 4) instead of two.  Per pixel at order 120: 6 nodes 8.9 ms, 14 nodes 17.4, 30 nodes 38.1, 53 nodes 55.9; groups
-// of 8 rows whatever the nodes took 12.1, 20.4, 38.1, 67.2, and one tile of 64 rows with its products staged in shared
-// memory (three barriers a step) 79.  Twice the row groups of half the rows were slower (6 nodes 10.0, 14 nodes 21.4)
-// but at exactly 8 nodes (11.9 against 12.2): each thread forms the products of its keys again for fewer rows.
-constexpr int w_rows(int rg, int r) { return r * rg + kWX + kWY + 1; }
+// R <= 4) instead of two.  Per pixel at order 120: 6 nodes 8.6 ms, 14 nodes 15.6, 30 nodes 32.7, 53 nodes 51.0; with
+// square tiles (8 x 16, 78 % of their keys in the triangle against 90; at order 42 52 % against 68) 8.9, 17.4, 38.1, 55.9;
+// groups of 8 rows whatever the nodes, on those, took 12.1, 20.4, 38.1, 67.2, and one tile of 64 rows with its products
+// staged in shared memory (three barriers a step) 79.  The cosines' row between the two x-blocks keeps their lanes off
+// each other's banks.  Twice the row groups of half the rows were slower (on square tiles 6 nodes 10.0, 14
+// nodes 21.4) but at exactly 8 nodes (11.9 against 12.2): each thread forms the products of its keys again for fewer rows.
+constexpr int w_rows(int rg, int r) { return r * rg + 2 * kWX + kWY + 1; }
 constexpr int w_blocks(int r) { return r <= 4 ? 4 : r <= 7 ? 3 : 2; }
 constexpr size_t w_smem(int rg, int r)
 {
@@ -116,10 +119,10 @@ __global__ void __launch_bounds__(kWThreads, w_blocks(R)) k_w_gemm(const int4 *_
                                                          int t0, double w0, double w1, int n_tau, long long n_keys,
                                                          double *__restrict__ Wraw)
 {
-    constexpr int QG = 8 / RG, NR = w_rows(RG, R);
-    extern __shared__ __align__(16) double wsm[];   // [stage][row: nodes, x ladder, y ladder, cos][point]
+    constexpr int QG = 8 / RG, NR = w_rows(RG, R), XC = R * RG + kWX, Y0 = XC + 1 + kWX;
+    extern __shared__ __align__(16) double wsm[];   // [stage][row: nodes, x ladder, cos, x ladder of the next block, y ladder][point]
     const int4 tl = tiles[blockIdx.x];
-    const int m = tl.x, x0 = tl.y, y0 = tl.z;
+    const int m = tl.x, x0 = tl.y, y0 = tl.z, na = tl.w;   // the tile's first na columns lie in the block x0, the others in the next
     const int L = n_max - m + 1;
     const int tid = threadIdx.x, tc = tid & 15, g = tid >> 4, rg = g % RG, qg = g / RG;
     const int nsteps = Qp / kWQ;
@@ -132,17 +135,17 @@ __global__ void __launch_bounds__(kWThreads, w_blocks(R)) k_w_gemm(const int4 *_
             if (row < R * RG) {
                 ok = row < n_nodes;
                 if (ok) src = bw + (size_t)row * Qp;
-            } else if (row < R * RG + kWX) {
-                const int x = x0 + row - R * RG;
-                ok = x <= L - 1;
-                if (ok) src = lad1 + (size_t)(m + 2 * x) * Qp;
-            } else if (row < R * RG + kWX + kWY) {
-                const int y = y0 + row - R * RG - kWX;
-                ok = y <= L - 1;
-                if (ok) src = lad2 + (size_t)(m + 2 * y) * Qp;
-            } else {
+            } else if (row == XC) {
                 ok = true;
                 src = cm + (size_t)m * Qp;
+            } else if (row < Y0) {
+                const int c = row - R * RG - (row > XC), x = x0 + c;
+                ok = x <= L - 1 && (c < kWX || na < kWY);
+                if (ok) src = lad1 + (size_t)(m + 2 * x) * Qp;
+            } else {
+                const int c = row - Y0, y = c < na ? y0 + c : c - na;
+                ok = y <= L - 1;
+                if (ok) src = lad2 + (size_t)(m + 2 * y) * Qp;
             }
             cp_async16(st + row * kWPitch + qq, src + (ok ? step * kWQ + qq : 0), ok);
         }
@@ -163,8 +166,8 @@ __global__ void __launch_bounds__(kWThreads, w_blocks(R)) k_w_gemm(const int4 *_
         if (k + kWStages - 1 < nsteps) issue(k + kWStages - 1, (k + kWStages - 1) % kWStages);
         asm volatile("cp.async.commit_group;\n" ::);
         const double *st = wsm + (size_t)(k % kWStages) * NR * kWPitch;
-        const double *pa = st + rg * R * kWPitch, *px = st + R * RG * kWPitch;
-        const double *py = st + (R * RG + kWX + tc) * kWPitch, *pc = st + (R * RG + kWX + kWY) * kWPitch;
+        const double *pa = st + rg * R * kWPitch, *px = st + (tc < na ? R * RG : XC + 1) * kWPitch;
+        const double *py = st + (Y0 + tc) * kWPitch, *pc = st + XC * kWPitch;
 #pragma unroll 2
         for (int qq = qg; qq < kWQ; qq += QG) {
             const double yc = __dmul_rn(py[qq], pc[qq]);
@@ -204,7 +207,7 @@ __global__ void __launch_bounds__(kWThreads, w_blocks(R)) k_w_gemm(const int4 *_
         if (row >= n_nodes) continue;
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-            const int x = x0 + c, y = y0 + tc;
+            const int x = (tc < na ? x0 : x0 + kWX) + c, y = tc < na ? y0 + tc : tc - na;
             if (x + y > L - 1) continue;
             const long long n = m + x + y, a = m + x, b = x;
             const long long key = n * (n + 1) * (n + 2) / 6 + a * (a + 1) / 2 + b;
@@ -250,8 +253,14 @@ extern "C" int exm_w_build(exm_ctx *ctx, int n_nodes, const double *s_nodes, int
         std::vector<int4> tiles;
         for (int m = 0; m <= n_max; ++m) {
             const int L = n_max - m + 1;
-            for (int x0 = 0; x0 < L; x0 += kWX)
-                for (int y0 = 0; x0 + y0 <= L - 1; y0 += kWY) tiles.push_back(make_int4(m, x0, y0, 0));
+            int x0 = 0, y0 = 0;   // the next column to be placed
+            while (x0 < L) {
+                const int na = std::min(kWY, L - x0 - y0);
+                tiles.push_back(make_int4(m, x0, y0, na));
+                if (na < kWY) x0 += kWX, y0 = kWY - na;
+                else y0 += kWY;
+                if (x0 + y0 >= L) x0 += kWX, y0 = 0;
+            }
         }
         const size_t nW = (size_t)n_nodes * n_tau * n_keys;
         dbuf d_s, d_c2p, d_s2p, d_ap, d_cg, d_wq, d_resp, d_scale, d_W, d_out, d_tiles, d_l1, d_l2, d_dph, d_cm, d_bw, d_bad;
