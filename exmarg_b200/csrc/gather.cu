@@ -459,7 +459,7 @@ __device__ __forceinline__ void process_run(const PlaneArgs &a, RunCtx &c, unsig
                 fb[u] = __uint_as_float((f & 0x7FFFFFu) | 0x3F800000u) - 1.f;
                 fd[u] = __uint_as_float(c.nx[u].y);
                 w[u] = __uint_as_float(c.nx[u].z);
-                wt[u] = w[u] < 0.f ? c.wr : 1.f;
+                wt[u] = (int)c.nx[u].z < 0 ? c.wr : 1.f;   // the bit: a draw's plane weight may be zero
             }
             next_group(c);
             // close the running template where another one begins
