@@ -243,7 +243,7 @@ struct RunCtx {
     int sh;                     // window offset of a tap = its o0 + sh (+ a row when the beta fractions carry)
     unsigned lim;               // the taps the windows serve have offsets below lim
     unsigned ckf;               // the node's beta fraction, 23-bit fixed point
-    float wr, lw;               // weight of a random draw and its logarithm
+    float wr, lw;               // weight of a random draw (a factor up to EXM_LW_FACTOR) and its logarithm
     int beg, end;               // the warp's sorted positions (whole groups)
     int tF, tL;                 // the templates at the two ends of this warp's taps (may be shared with
     unsigned eF, eL;            // neighbouring warps): their partials go to this warp's edge slots (m, S)
@@ -413,7 +413,14 @@ __device__ __forceinline__ void open_edge(RunCtx &c, unsigned eo)
     __syncwarp();
 }
 
-template <bool BND, int PF, typename TE>
+// The draws' weight enters as a factor exp(lw) of their exponentials, outside the running maximum: one fused
+// multiply-add a tap.  That holds while the factor and its products with the exponentials stay within float32:
+// with |lw| <= EXM_LW_FACTOR what underflows (below 2^-126 of the largest unweighted value) is less than
+// 2^-126 e^60 = 1.3e-12 of the sum.  LOGW, for any other weight, adds lw to the tap's value, so that the maximum
+// includes it.
+#define EXM_LW_FACTOR 60.0
+
+template <bool BND, int PF, typename TE, bool LOGW>
 __device__ __forceinline__ void process_run(const PlaneArgs &a, RunCtx &c, unsigned &n_slow)
 {
     // the warp's positions walked in chunks of 128 ng; lane l takes the chunk's groups l ng + g, tap u of it
@@ -459,7 +466,8 @@ __device__ __forceinline__ void process_run(const PlaneArgs &a, RunCtx &c, unsig
                 fb[u] = __uint_as_float((f & 0x7FFFFFu) | 0x3F800000u) - 1.f;
                 fd[u] = __uint_as_float(c.nx[u].y);
                 w[u] = __uint_as_float(c.nx[u].z);
-                wt[u] = (int)c.nx[u].z < 0 ? c.wr : 1.f;   // the bit: a draw's plane weight may be zero
+                // the bit: a draw's plane weight may be zero
+                wt[u] = (int)c.nx[u].z < 0 ? (LOGW ? c.lw : c.wr) : (LOGW ? 0.f : 1.f);
             }
             next_group(c);
             // close the running template where another one begins
@@ -479,6 +487,7 @@ __device__ __forceinline__ void process_run(const PlaneArgs &a, RunCtx &c, unsig
             for (int u = 0; u < EXM_GT; ++u) {
                 interp_window<TE>((const TE *)(exm_gsm + c.s0), (const TE *)(exm_gsm + c.s1), o[u], fb[u], fd[u],
                                   fabsf(w[u]), c.sc, B[u], E[u]);
+                if (LOGW) E[u] += wt[u];
                 const float v = B[u] + E[u];
                 if (fast[u]) m = fmaxf(m, v);
                 if (PF == 1 && u == 1) __syncwarp();   // two taps' window reads in flight, for shapes with few registers
@@ -487,7 +496,7 @@ __device__ __forceinline__ void process_run(const PlaneArgs &a, RunCtx &c, unsig
 #pragma unroll
             for (int u = 0; u < EXM_GT; ++u) {
                 const float x = ex2_approx(((B[u] - m) + E[u]) * EXM_L2E);
-                if (fast[u]) S = fmaf(x, wt[u], S);
+                if (fast[u]) S = LOGW ? S + x : fmaf(x, wt[u], S);
             }
             cm = m;
             cS = S;
@@ -573,7 +582,7 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar)
 // only after pair p is done everywhere).  So at most two consecutive pairs are in flight, and the
 // consumers' accumulators alternate with the pair's parity (two warps in different pairs never
 // share a word), while the producer folds edges into a third set of its own.
-template <int NW, int PF, typename TE>
+template <int NW, int PF, typename TE, bool LOGW>
 __global__ void __launch_bounds__(NW * 32, 1) k_gather_planes(const __grid_constant__ CUtensorMap tmap,
                                                                 const __grid_constant__ PlaneArgs a)
 {
@@ -789,9 +798,9 @@ __global__ void __launch_bounds__(NW * 32, 1) k_gather_planes(const __grid_const
                 rc.s1 = ((p + 1) % 3) * SLOT_B;
                 rc.acc = acc_o + 4u * (2u * (p & 1) * tch);
                 if (bnd)
-                    process_run<true, PF, TE>(a, rc, n_slow);
+                    process_run<true, PF, TE, LOGW>(a, rc, n_slow);
                 else
-                    process_run<false, PF, TE>(a, rc, n_slow);
+                    process_run<false, PF, TE, LOGW>(a, rc, n_slow);
             }
             __syncwarp();
             mbar_arrive(&done[p & 1]);
@@ -842,16 +851,20 @@ struct GatherCfg {
 static const GatherCfg kGatherCfgs[] = {{20, 2}, {28, 1}, {16, 2}, {24, 2}, {24, 1}};
 static const int kNumGatherCfgs = (int)(sizeof(kGatherCfgs) / sizeof(kGatherCfgs[0]));
 
-template <int NW, int PF, typename TE>
+template <int NW, int PF, typename TE, bool LOGW = false>
 static void launch_planes(exm_ctx *ctx, const PlaneArgs &a, dim3 grid, size_t smem)
 {
-    exm_allow_smem(ctx, (const void *)k_gather_planes<NW, PF, TE>, smem);
-    k_gather_planes<NW, PF, TE><<<grid, NW * 32, smem, ctx->stream>>>(ctx->tmap, a);
+    exm_allow_smem(ctx, (const void *)k_gather_planes<NW, PF, TE, LOGW>, smem);
+    k_gather_planes<NW, PF, TE, LOGW><<<grid, NW * 32, smem, ctx->stream>>>(ctx->tmap, a);
 }
 
 template <typename TE>
 static void launch_cfg_t(exm_ctx *ctx, int cfg, const PlaneArgs &a, dim3 grid, size_t smem)
 {
+    if (!(std::fabs((double)a.lw) <= EXM_LW_FACTOR)) {   // weights given by the caller: one shape is enough
+        launch_planes<20, 2, TE, true>(ctx, a, grid, smem);
+        return;
+    }
     switch (cfg) {
     case 0: launch_planes<20, 2, TE>(ctx, a, grid, smem); break;
     case 1: launch_planes<28, 1, TE>(ctx, a, grid, smem); break;

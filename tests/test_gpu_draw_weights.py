@@ -1,5 +1,6 @@
 """The importance weight of the random draws in the plane gather: a draw keeps its weight whatever its phase (equal
-phases in both detectors give it a plane weight of exactly zero), on the staged windows and on the exact path.
+phases in both detectors give it a plane weight of exactly zero) and whatever log weight the caller gives, on the staged
+windows and on the exact path.
 exm_node_values against the float64 oracle on the same float32 trajectories and times."""
 
 import numpy as np
@@ -64,3 +65,23 @@ def test_a_draw_of_equal_phases_keeps_its_weight(dtype, phases, path):
     geo = restate.node_geometry(store.s, store.alpha_lo, store.alpha_hi, bank.u, 0.1267)
     want = restate.node_values(traj, store, geo, [list(range(NODES))], (sel, lw))
     _check(got, want, _tolerance(store))
+
+
+@pytest.mark.parametrize("lw", [-200.0, -90.0, -61.0, 60.0, 61.0, 95.0, 200.0])
+@pytest.mark.parametrize("draws", ["all", "half"])
+@pytest.mark.parametrize("dtype, path", [("f32", "windows"), ("f32", "exact"), ("f16", "windows")])
+def test_any_log_weight(lw, draws, dtype, path):
+    nm, walk = 40, 300
+    store, bank, traj, rng = _case(nm, 5, 200, 219, NODES, 12)
+    if path == "exact":
+        traj["lqL"] += rng.uniform(-14.0, 14.0, traj["lqL"].shape).astype(np.float32)
+    sel = np.sort(np.stack([rng.choice(NT, walk, replace=False) for _ in range(nm)]), axis=1).astype(np.int32)
+    drawn = np.ones(sel.shape, bool) if draws == "all" else rng.random(sel.shape) < 0.5
+    times = (sel, np.where(drawn, np.float32(lw), np.float32(0.0)))
+    store_d = eb.with_table_dtype(store, dtype) if dtype != "f32" else store
+    got, _ = _node_values(store_d, bank, traj, times)
+    store.tables = [eb.quantize_table(T, dtype)[0] for T in store.tables]
+    geo = restate.node_geometry(store.s, store.alpha_lo, store.alpha_hi, bank.u, 0.1267)
+    want = restate.node_values(traj, store, geo, [list(range(NODES))], times)
+    # and two roundings of a float32 sum of the weight and the interpolation term
+    _check(got, want, _tolerance(store) + 2 * 2.0 ** -24 * (abs(lw) + 10.0))
