@@ -63,7 +63,7 @@ struct PlaneArgs {
     int stage;                   // 1: stage the planes; 0 (the wait-expiry test): no copy is issued, so the
                                  // first wait runs out and the kernel returns its timeout status
     int cki[EXM_MAX_NODES];
-    unsigned ckf[EXM_MAX_NODES];  // fraction of a node's beta shift, 23-bit fixed point
+    float ckf[EXM_MAX_NODES];    // fraction of a node's beta shift
     float tsc[EXM_MAX_NODES];    // per node: value = tsc * stored element
 };
 
@@ -225,6 +225,10 @@ __device__ __forceinline__ void interp_window(const TE *s0, const TE *s1, int o,
     }
 }
 
+// -1 where the sum f of a tap's and a node's beta fractions stays below 1, 0 where it carries into the row: by the bits,
+// since with four more predicates the tap loop spills (2048 templates x 53 nodes 62.8 ms, this 61.5)
+__device__ __forceinline__ int no_carry(float f) { return ((int)__float_as_uint(f) - 0x3F800000) >> 31; }
+
 // One run of tap descriptors (sorted by template, in groups of EXM_GT taps of one template) on the
 // two staged planes of pair p.  Each lane takes ng consecutive groups of a chunk; a template that
 // lies inside one lane's groups is merged into its accumulator by that lane, one that spans lanes
@@ -232,17 +236,16 @@ __device__ __forceinline__ void interp_window(const TE *s0, const TE *s1, int o,
 // byte offsets below are into exm_gsm
 struct RunCtx {
     const uint4 *descr;
-    const int32_t *tsr;
     unsigned s0, s1;            // the staged windows of planes p and p + 1 (element type TE)
     float sc;                   // the node's scale (16-bit tables)
     unsigned acc, accst;        // accumulator set of the run's templates (m at acc + 4 t; S at + accst)
     unsigned bsh, bcf;          // boundary blocks: per-template window offset (int; EXM_BSH_NONE for templates
-                                // whose boundary point is not this node) and beta fraction (23-bit fixed point)
+                                // whose boundary point is not this node) and beta fraction
     int ng;                     // groups per lane and chunk
-    int lo, m_base, n, k, r;
+    int dm, n, k, r;            // block-local template = descriptor's + dm
     int sh;                     // window offset of a tap = its o0 + sh (+ a row when the beta fractions carry)
     unsigned lim;               // the taps the windows serve have offsets below lim
-    unsigned ckf;               // the node's beta fraction, 23-bit fixed point
+    float ckf;                  // the node's beta fraction
     float wr, lw;               // weight of a random draw (a factor up to EXM_LW_FACTOR) and its logarithm
     int beg, end;               // the warp's sorted positions (whole groups)
     int tF, tL;                 // the templates at the two ends of this warp's taps (may be shared with
@@ -317,7 +320,7 @@ __device__ __forceinline__ void split_double(double v, float &m, float &S)
 // computes them 32 at a time instead of stalling the warp on one lane's float64 path; those a full queue
 // cannot take are computed here and merged into the lane's running partial
 template <bool BND, typename TE>
-__device__ __forceinline__ void slow_group(const PlaneArgs &a, const RunCtx &c, int pj, int t, int sh, unsigned ckf,
+__device__ __forceinline__ void slow_group(const PlaneArgs &a, const RunCtx &c, int pj, int t, int sh, float ckf,
                                            float &m, float &S, unsigned &n_slow)
 {
     const int lane = threadIdx.x & 31;
@@ -328,7 +331,7 @@ __device__ __forceinline__ void slow_group(const PlaneArgs &a, const RunCtx &c, 
         uint4 q = make_uint4(0u, 0u, 0u, EXM_DESC_PAD);
         if (t >= 0) {
             q = __ldg(c.descr + pj);
-            const int o = ((int)q.w >> 13) + sh + (int)((q.x + ckf) >> 23) * TabElem<TE>::wd;
+            const int o = ((int)q.w >> 13) + sh + (~no_carry(__uint_as_float(q.x) + ckf) & TabElem<TE>::wd);
             sl = (unsigned)o >= c.lim && (int)q.w >= EXM_DESC_REAL;
         }
         const unsigned bal = __ballot_sync(0xffffffffu, sl);
@@ -342,7 +345,7 @@ __device__ __forceinline__ void slow_group(const PlaneArgs &a, const RunCtx &c, 
             if (pos < EXM_SLOWQ) {
                 ((int2 *)(exm_gsm + c.q))[pos] = make_int2(pj, il | (int)((q.z >> 31) << 29));
             } else {
-                double v = slow_tap<BND, TE>(a, il, c.tsr[pj], c.k, c.r, c.m_base, c.sc);
+                double v = slow_tap<BND, TE>(a, il, a.tside[(c.r - a.r0) * a.per_lag + pj], c.k, c.r, a.m_base, c.sc);
                 if (q.z >> 31) v += (double)c.lw;
                 float m2, S2;
                 split_double(v, m2, S2);
@@ -359,7 +362,7 @@ __device__ __forceinline__ void slow_group(const PlaneArgs &a, const RunCtx &c, 
 // the template of the descriptor at sorted position j (block-local)
 __device__ __forceinline__ int desc_template(const RunCtx &c, int j)
 {
-    return (int)(__ldg(&c.descr[exm_desc_phys(j, c.ng)].w) & 0x1FFFu) + c.m_base - c.lo;
+    return (int)(__ldg(&c.descr[exm_desc_phys(j, c.ng)].w) & 0x1FFFu) + c.dm;
 }
 
 // this warp's share [c.beg, c.end) of the pair's run [beg, end): whole storage chunks per warp, as evenly as
@@ -434,20 +437,20 @@ __device__ __forceinline__ void process_run(const PlaneArgs &a, RunCtx &c, unsig
 #pragma unroll 1
         for (int g = 0; g < ng; ++g) {
             // the group's template (-1: nothing to do) and the window shift of its taps
-            int t = (int)(c.nx[0].w & 0x1FFFu) + c.m_base - c.lo;
+            int t = (int)(c.nx[0].w & 0x1FFFu) + c.dm;
             if (!c.in) t = -1;
             if (t >= c.n) {   // outside the block's templates: report and skip
                 atomicOr(a.err, EXM_DEVERR_BOUNDS);
                 t = -1;
             }
             int sh = c.sh;
-            unsigned ckf = c.ckf;
+            float ckf = c.ckf;
             if (BND) {
                 sh = EXM_BSH_NONE;
-                ckf = 0u;
+                ckf = 0.f;
                 if (t >= 0) {
                     sh = ((const int *)gsm_f(c.bsh))[t];
-                    ckf = ((const unsigned *)gsm_f(c.bcf))[t];
+                    ckf = gsm_f(c.bcf)[t];
                 }
                 if (sh == EXM_BSH_NONE) t = -1;
             }
@@ -458,12 +461,13 @@ __device__ __forceinline__ void process_run(const PlaneArgs &a, RunCtx &c, unsig
             bool sl = false;
 #pragma unroll
             for (int u = 0; u < EXM_GT; ++u) {
-                const unsigned f = c.nx[u].x + ckf;
-                const int ou = ((int)c.nx[u].w >> 13) + sh + (int)(f >> 23) * WD;
+                const float f = __uint_as_float(c.nx[u].x) + ckf;   // the fractions carry into the row
+                const int nc = no_carry(f);
+                const int ou = ((int)c.nx[u].w >> 13) + sh + (~nc & WD);
                 fast[u] = (unsigned)ou < c.lim;
                 sl = sl || (!fast[u] && (int)c.nx[u].w >= EXM_DESC_REAL);
                 o[u] = fast[u] ? ou : lane;
-                fb[u] = __uint_as_float((f & 0x7FFFFFu) | 0x3F800000u) - 1.f;
+                fb[u] = f - __uint_as_float(~nc & 0x3F800000);
                 fd[u] = __uint_as_float(c.nx[u].y);
                 w[u] = __uint_as_float(c.nx[u].z);
                 // the bit: a draw's plane weight may be zero
@@ -639,7 +643,7 @@ __global__ void __launch_bounds__(NW * 32, 1) k_gather_planes(const __grid_const
         }
         if (bnd) {
             int bs = EXM_BSH_NONE;
-            unsigned bf = 0u;
+            float bf = 0.f;
             if (a.bnode[lo + j] == k) {
                 const double cbv = a.cb[lo + j];
                 const double f = floor(cbv);
@@ -647,11 +651,11 @@ __global__ void __launch_bounds__(NW * 32, 1) k_gather_planes(const __grid_const
                 bs = EXM_BSH_FAR;   // no tap reaches the window: every one takes the exact path
                 if (abs(rows) <= EXM_MAX_SHIFT) {
                     bs = rows * TabElem<TE>::wd;
-                    bf = __double2uint_rn((cbv - f) * 8388608.0);
+                    bf = (float)(cbv - f);
                 }
             }
             ((int *)gsm_f(bsh_o))[j] = bs;
-            ((unsigned *)gsm_f(bcf_o))[j] = bf;
+            gsm_f(bcf_o)[j] = bf;
         }
     }
     if (tid == 0) {
@@ -749,13 +753,11 @@ __global__ void __launch_bounds__(NW * 32, 1) k_gather_planes(const __grid_const
         const int *offr = a.off + (long long)rl * EXM_NPAIR * (a.nmc + 1);
         RunCtx rc;
         rc.descr = a.desc + (long long)rl * a.per_lag;
-        rc.tsr = a.tside + (long long)rl * a.per_lag;
         rc.bsh = bsh_o;
         rc.bcf = bcf_o;
         rc.accst = 4u * tch;
         rc.ng = a.ng;
-        rc.lo = lo;
-        rc.m_base = a.m_base;
+        rc.dm = a.m_base - lo;
         rc.n = n;
         // rows 0 .. up of the window are served: up + 1 must be in the window, and the table's last row
         // pair, where the reference clamps beta just below the top, is left to the exact path
@@ -1005,7 +1007,7 @@ void exm_run_gather_planes(exm_ctx *ctx, exm_slot &sl, const ChunkInfo &ci, int 
     for (int k = 0; k < ctx->nn; ++k) {
         const double f = std::floor(ctx->ck[k]);
         a.cki[k] = (int)f;
-        a.ckf[k] = (unsigned)std::nearbyint((ctx->ck[k] - f) * 8388608.0);
+        a.ckf[k] = (float)(ctx->ck[k] - f);
         a.tsc[k] = ctx->tscale[k];
     }
     int maxn = 0;

@@ -101,8 +101,8 @@ struct TapGeom {
 
 // The per-tap quantities that do not depend on the node (the reference computes
 // them per node, exmarg/search/gather.py:50-82): the plane pair p and the weight w
-// of plane p + 1, beta-hat = ln|z_L| 2/dbeta - ln(u)/dbeta as floor + fraction (23-bit fixed point,
-// rounded: 2^23 carries into the row when a node's fraction is added), and the Delta coordinate of the unclamped-beta case as (d0, fd).
+// of plane p + 1, beta-hat = ln|z_L| 2/dbeta - ln(u)/dbeta as floor + fraction (a float32, 1 where it rounds up: the
+// gather carries it into the row), and the Delta coordinate of the unclamped-beta case as (d0, fd).
 // ln|z| enters as its float32 value plus the filter's float32 residual (llo, hlo: ln|z| - float(ln|z|), zero for
 // trajectories given as float32), so beta-hat and Delta see the filter's float64 value; the phases stay float32
 // and are subtracted in float32, as the reference does.
@@ -124,18 +124,18 @@ __device__ __forceinline__ void exm_tap_phase(float phL, float phH, const TapGeo
     }
 }
 
-__device__ __forceinline__ void exm_tap_beta(float lqL, float lqLlo, double boff, const TapGeom &g, int &ib, unsigned &fb)
+__device__ __forceinline__ void exm_tap_beta(float lqL, float lqLlo, double boff, const TapGeom &g, int &ib, float &fb)
 {
     const double bh = ((double)lqL + (double)lqLlo) * g.rdb + boff;
     const double fl = floor(bh);
     ib = (int)fmax(fmin(fl, 1023.0), -1024.0);
-    fb = __double2uint_rn((bh - fl) * 8388608.0);
+    fb = (float)(bh - fl);
 }
 
 __device__ __forceinline__ int exm_tap_row(float lqL, float lqLlo, double boff, const TapGeom &g)
 {
     int ib;
-    unsigned fb;
+    float fb;
     exm_tap_beta(lqL, lqLlo, boff, g, ib, fb);
     return ib;
 }

@@ -4,7 +4,7 @@
 // p + 1, beta-hat and the Delta coordinate do not depend on the node, so they are
 // computed once per tap (in float64, as the reference computes them per node) and
 // packed into 16 bytes:
-//   x = fraction of beta-hat (23-bit fixed point), y = fd (float, fraction of Delta),
+//   x = fraction of beta-hat (float), y = fd (float, fraction of Delta),
 //   z = w (float, weight of plane p + 1) | bit 31: the time is a random draw,
 //   w = window offset (19 bits, signed) << 13 | template (13 bits),
 // with the staging windows already placed (k_windows runs between the count and the
@@ -300,12 +300,12 @@ __global__ void __launch_bounds__(256) k_tap_scatter(TapArgs a)
                     const int pos = base[p[m]] + wcnt[m][warp][p[m]] + rk[m];
                     const WalkEntry e = w[k0 - c0 + m * 256 + tid];
                     int ib;
-                    unsigned fb;
+                    float fb;
                     exm_tap_beta(e.x, e.lo, boff, a.g, ib, fb);
                     const int rd = d0[m] - C0, rb0 = ib - Rh;
                     const bool far = (unsigned)rd > (unsigned)(a.wd - 2) || rb0 < -1024 || rb0 > 1023;
                     if (pos >= 0 && pos < a.pitch) {   // sorted order; k_tap_order rearranges each chunk afterwards
-                        desc[pos] = make_uint4(fb, __float_as_uint(fd[m]),
+                        desc[pos] = make_uint4(__float_as_uint(fb), __float_as_uint(fd[m]),
                                                __float_as_uint(wp[m]) | ((unsigned)e.t & 0x80000000u),
                                                ((unsigned)(far ? EXM_O_FAR : rb0 * a.wd + rd) << 13) | (unsigned)i);
                         tside[pos] = e.t & 0x7FFFFFFF;
