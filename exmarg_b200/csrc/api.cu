@@ -654,7 +654,7 @@ extern "C" int exm_bank_set(exm_ctx *ctx, int nm, int nfreq, int lo, int n_time,
     for (int m = 0; m < nm; ++m) REQUIRE(u[m] > 0, EXM_ERR_ARG, "template powers u must be positive");
     ctx->bank_ok = true;
     ctx->prep_ok = false;
-    ctx->traj_ok = ctx->times_ok = false;
+    ctx->traj_ok = ctx->times_ok = ctx->ran_ok = false;
     API_END(ctx)
 }
 
@@ -1152,11 +1152,49 @@ extern "C" int exm_pe_intrinsic(exm_ctx *ctx, int n_seg, const double *d_H, cons
         for (int i = 0; i < ctx->nm; ++i) ln_lambda[(size_t)e * ctx->nm + ctx->order[i]] = lnl[i];
     }
     ctx->traj_ok = ctx->times_ok = false;
-    ctx->last_shape_ok = n_seg > 0;
+    ctx->ran_ok = n_seg > 0;
     API_END(ctx)
 }
 
 // ------------------------------------------------------------------ autotuner
+
+// Times and descriptors for the autotuner's shape, from the trajectories in the slot (the last segment's, or those of a
+// later stage call).  They are always built anew: the filter and the trajectory upload share the descriptors' memory, and
+// the stage calls build descriptors of other shapes.  The caller's times are kept: walked if they are of this shape, else
+// put back after the build.
+static void tune_taps(exm_ctx *ctx, exm_slot &sl, const RunShape &rs, const ChunkInfo &ci)
+{
+    const size_t nm = ctx->nm;
+    const bool had_lo = sl.trajlo.p != nullptr;
+    const bool own = ctx->times_ok && ctx->cur_nwalk == rs.nwalk, times = ctx->times_ok;
+    const bool draw = rs.K > 0 && !own;
+    std::vector<int32_t> keep;
+    if (draw && times) {
+        keep.resize(nm * ctx->cur_nwalk);
+        EXM_CUDA(cudaMemcpyAsync(keep.data(), sl.sel.p, sizeof(int32_t) * keep.size(), cudaMemcpyDeviceToHost,
+                                 ctx->stream));
+        EXM_CUDA(cudaStreamSynchronize(ctx->stream));
+        ctx->times_ok = false;   // until they are back
+    }
+    ensure_slot(ctx, sl, rs);
+    if (ctx->traj_fp64 && !had_lo) EXM_CUDA(cudaMemsetAsync(sl.trajlo.p, 0, sl.trajlo.bytes, ctx->stream));
+    if (draw) {
+        uint64_t *w = (uint64_t *)((double *)sl.hostin.p + 6 * (size_t)ctx->nfreq);
+        exm_pcg_words(0, w);
+        EXM_CUDA(cudaMemcpyAsync((void *)state_words(ctx, sl), w, 4 * sizeof(uint64_t), cudaMemcpyHostToDevice,
+                                 ctx->stream));
+        exm_run_pcg(ctx, sl, state_words(ctx, sl), rs.K, rs.S);
+        exm_run_topk(ctx, sl, ctx->nm, (const int *)ctx->d_order.p, rs.K, rs.S);
+    }
+    EXM_CUDA(cudaMemsetAsync(sl.dev_err.p, 0, sizeof(unsigned), ctx->stream));
+    exm_run_taps(ctx, sl, ci, 0, ctx->ntau, true);
+    if (draw && times) {
+        EXM_CUDA(cudaMemcpyAsync(sl.sel.p, keep.data(), sizeof(int32_t) * keep.size(), cudaMemcpyHostToDevice,
+                                 ctx->stream));
+        EXM_CUDA(cudaStreamSynchronize(ctx->stream));
+        ctx->times_ok = true;
+    }
+}
 
 extern "C" int exm_autotune(exm_ctx *ctx, int n_loud, int n_random, int reps, int *best_cfg, int *best_chunk_pct,
                             double *ms_per_cfg)
@@ -1164,12 +1202,13 @@ extern "C" int exm_autotune(exm_ctx *ctx, int n_loud, int n_random, int reps, in
     API_BEGIN(ctx)
     EXM_CUDA(cudaSetDevice(ctx->dev));
     REQUIRE(ctx->prep_ok, EXM_ERR_STATE, "exm_pe_prepare first");
-    REQUIRE(ctx->last_shape_ok, EXM_ERR_STATE, "run exm_pe_intrinsic once first (the autotuner replays its last segment)");
+    REQUIRE(ctx->ran_ok, EXM_ERR_STATE, "run exm_pe_intrinsic on this bank once first (the autotuner times the gather on its data)");
     const RunShape rs = run_shape(ctx, n_loud, n_random);
     REQUIRE(rs.nmc_max >= ctx->nm && rs.rc >= ctx->ntau, EXM_ERR_ARG,
             "the autotuner needs the whole bank and every lag in one gather (bank <= 8192 templates)");
     exm_slot &sl = ctx->slot;
     ChunkInfo ci{0, ctx->nm, rs.nwalk, rs.use_sel, rs.lw};
+    tune_taps(ctx, sl, rs, ci);
     const int n = exm_gather_num_cfgs();
     cudaEvent_t e0, e1;
     EXM_CUDA(cudaEventCreate(&e0));

@@ -185,7 +185,8 @@ struct exm_ctx {
 
     // current segment state for the stage entry points
     exm_slot slot;
-    bool traj_ok = false, times_ok = false, last_shape_ok = false;
+    bool traj_ok = false, times_ok = false;
+    bool ran_ok = false;              // exm_pe_intrinsic has run on this bank: the slot holds trajectories of it
     int cur_nwalk = 0;
     float cur_lw = 0.f;
     std::vector<exm_slot> slots;

@@ -257,8 +257,9 @@ EXM_API int exm_pe_intrinsic(exm_ctx *ctx, int n_seg, const double *d_H, const d
                      double *ln_b);
 
 /* Autotuner of the plane gather's launch shape (warps per block x taps per register
- * group): replays the gather of the last segment analysed by exm_pe_intrinsic on this
- * context (same n_loud, n_random) once per shape, times each with CUDA events (reps
+ * group): after exm_pe_intrinsic on this context's bank, runs the gather of n_loud, n_random on
+ * the trajectories the context holds (the last segment's, or a later exm_filter's or
+ * exm_set_trajectories') once per shape, times each with CUDA events (reps
  * launches), keeps the fastest for later calls and writes its index to best_cfg and the
  * ms per launch of every shape to ms_per_cfg (if not NULL; room for 16 entries: this build
  * has 5 shapes, warps per block including the producer warp x pairs of taps whose window reads
