@@ -866,36 +866,131 @@ extern "C" int exm_pe_prepare(exm_ctx *ctx, double ymin, int prior, const double
 // ------------------------------------------------------------------ the per-segment pipeline
 
 struct RunShape {
-    int K, S, nwalk, use_sel, nmc_max, rc, nparts;
+    int K, S, nwalk, use_sel, nmc_max;
+    int rc_cap, rc, nparts;   // lags per pass, by their taps and by what the budget holds; parts of the plane pairs
     float lw;
 };
 
-// lags per pass (descriptors and time indices of at most 8 GiB) and parts of the plane pairs per block
-static void plan_lags(exm_ctx *ctx, RunShape &rs)
+// what the sizes of the workspace depend on
+struct SlotDims {
+    int nm, nt, nf, nn, ntau, sm_count;
+    bool lo;   // residuals of ln|z| are kept
+};
+
+static SlotDims slot_dims(const exm_ctx *ctx)
 {
-    const size_t per_lag = (size_t)rs.nmc_max * rs.nwalk * 20;
-    const size_t cap = (size_t)8 << 30;
-    rs.rc = (int)std::max<size_t>(1, std::min<size_t>((size_t)ctx->ntau, cap / std::max<size_t>(per_lag, 1)));
-    rs.nparts = exm_gather_parts(ctx, rs.nmc_max, 0, rs.nwalk, rs.rc);
+    return {ctx->nm, ctx->nt, ctx->nfreq, ctx->nn, ctx->ntau, ctx->sm_count, ctx->traj_fp64};
 }
 
-// the buffers of the tap build and the gather
-static void ensure_taps(exm_ctx *ctx, exm_slot &sl, const RunShape &rs)
+struct SlotNeed {
+    dbuf exm_slot::*buf;
+    size_t bytes;
+};
+
+// lags per pass: descriptors and time indices of at most 8 GiB, without the padding of their runs (up to 3 entries for each
+// of a template's 48 plane pairs: 7 % at 2048 walked times, 72 % at 200)
+static int lags_by_taps(int nmc, int nwalk, int ntau)
+{
+    const size_t per_lag = (size_t)nmc * nwalk * 20, cap = (size_t)8 << 30;
+    return (int)std::max<size_t>(1, std::min<size_t>((size_t)ntau, cap / std::max<size_t>(per_lag, 1)));
+}
+
+static void plan_lags(exm_ctx *ctx, RunShape &rs)
+{
+    rs.rc_cap = rs.rc = lags_by_taps(rs.nmc_max, rs.nwalk, ctx->ntau);
+    rs.nparts = exm_gather_parts(ctx, rs.nmc_max, 0, rs.rc);
+}
+
+// the buffers of the tap build, the gather and the node values
+static std::vector<SlotNeed> tap_needs(const SlotDims &d, const RunShape &rs)
 {
     const size_t pitch = (size_t)exm_desc_pitch(rs.nmc_max, rs.nwalk);
     // offsets, and the counts of the parts of the walked times (the parts of a smaller last pass: 32 at most)
     size_t parts = 0;
-    for (int nmc : {rs.nmc_max, ctx->nm % rs.nmc_max})
-        for (int rc : {rs.rc, ctx->ntau % rs.rc}) {
+    for (int nmc : {rs.nmc_max, d.nm % rs.nmc_max})
+        for (int rc : {rs.rc, d.ntau % rs.rc}) {
             if (nmc <= 0 || rc <= 0) continue;
-            const int nq = exm_tap_parts(ctx, nmc, rs.nwalk, rc);
+            const int nq = exm_tap_parts(d.sm_count, nmc, rs.nwalk, rc);
             if (nq > 1) parts = std::max(parts, (size_t)nq * rc * nmc);
         }
-    exm_ensure(ctx, sl.cnt, EXM_NPAIR * ((size_t)rs.rc * (rs.nmc_max + 1) + parts) * sizeof(int));
-    exm_ensure(ctx, sl.desc, (size_t)rs.rc * pitch * sizeof(uint4));
-    exm_ensure(ctx, sl.tside, (size_t)rs.rc * pitch * sizeof(int32_t));
-    exm_ensure(ctx, sl.part, (size_t)(ctx->nn + 1) * ctx->ntau * rs.nparts * ctx->nm * sizeof(double));
+    return {{&exm_slot::cnt, EXM_NPAIR * ((size_t)rs.rc * (rs.nmc_max + 1) + parts) * sizeof(int)},
+            {&exm_slot::desc, (size_t)rs.rc * pitch * sizeof(uint4)},
+            {&exm_slot::tside, (size_t)rs.rc * pitch * sizeof(int32_t)},
+            {&exm_slot::part, (size_t)(d.nn + 1) * d.ntau * rs.nparts * d.nm * sizeof(double)},
+            {&exm_slot::lamN, (size_t)(d.nn + 1) * d.nm * sizeof(double)}};
+}
+
+// every device buffer of a slot
+static std::vector<SlotNeed> slot_needs(const SlotDims &d, const RunShape &rs)
+{
+    std::vector<SlotNeed> v = tap_needs(d, rs);
+    const size_t nmc = rs.nmc_max, nt = d.nt, nf = d.nf, nm = d.nm;
+    for (SlotNeed &n : v)   // the filter's buffer before it holds descriptors
+        if (n.buf == &exm_slot::desc) n.bytes = std::max(n.bytes, 2 * nmc * nt * sizeof(double2));
+    const size_t n_draws = rs.K > 0 ? ((nm * rs.S + EXM_MAX_REJ + 63) / 64) * 64 : 0;
+    const SlotNeed more[] = {
+        {&exm_slot::traj, 2 * nmc * nt * sizeof(float2)},
+        {&exm_slot::trajlo, d.lo ? 2 * nmc * nt * sizeof(float) : 0},
+        {&exm_slot::keys, std::max<size_t>(rs.K > 0 ? nmc * nt : 1, n_draws) * sizeof(uint32_t)},
+        {&exm_slot::picks, std::max<size_t>(1, nm * rs.S) * sizeof(int32_t)},
+        {&exm_slot::rej, (1 + EXM_MAX_REJ) * sizeof(int)},
+        {&exm_slot::sel, std::max<size_t>(1, rs.use_sel ? nmc * rs.nwalk : 1) * sizeof(int32_t)},
+        {&exm_slot::hist, (EXM_HB_N + 256) * sizeof(int)},
+        {&exm_slot::win, (2 + EXM_MAX_NODES) * sizeof(int)},
+        {&exm_slot::lnl, nm * sizeof(double)},
+        {&exm_slot::lnb, sizeof(double)},
+        {&exm_slot::dev_err, sizeof(unsigned)},
+        {&exm_slot::din, 6 * nf * sizeof(double) + 2 * nf * sizeof(float2) + 4 * sizeof(uint64_t)}};
+    v.insert(v.begin(), std::begin(more), std::end(more));
+    return v;
+}
+
+// The slot's buffers for a shape.  Where the budget (or the device) does not hold the descriptors of all the pass's lags
+// beside the rest, the pass takes fewer: the partial sums of a lag are its own.
+static void ensure_needs(exm_ctx *ctx, exm_slot &sl, RunShape &rs, std::vector<SlotNeed> (*needs)(const SlotDims &, const RunShape &))
+{
+    const SlotDims d = slot_dims(ctx);
+    std::vector<SlotNeed> v = needs(d, rs);
+    auto missing = [&]() {
+        size_t m = 0;
+        for (const SlotNeed &n : v) m += std::max(n.bytes, (sl.*n.buf).bytes) - (sl.*n.buf).bytes;
+        return m;
+    };
+    if (missing() > 0) {
+        size_t fr = 0, tot = 0;
+        EXM_CUDA(cudaMemGetInfo(&fr, &tot));
+        const size_t left = std::min(fr, ctx->budget - ctx->used);
+        while (missing() > left && (rs.nparts > 1 || rs.rc > 1)) {
+            if (rs.nparts > 1)
+                rs.nparts /= 2;
+            else
+                rs.rc -= std::max(1, rs.rc / 8);
+            v = needs(d, rs);
+        }
+    }
+    for (const SlotNeed &n : v)
+        if (n.bytes) exm_ensure(ctx, sl.*n.buf, n.bytes);
     sl.nparts = rs.nparts;
+}
+
+static void ensure_taps(exm_ctx *ctx, exm_slot &sl, RunShape &rs) { ensure_needs(ctx, sl, rs, tap_needs); }
+
+// device bytes that exm_pe_intrinsic takes for a bank on the store of ctx, beside the store: the slot, the bank's arrays
+// and cuFFT's work area (about the rows it transforms)
+size_t exm_workspace_bytes(const exm_ctx *ctx, int nm, int nt, int nfreq, int K, int S)
+{
+    RunShape rs{};
+    rs.K = K;
+    rs.S = K > 0 ? S : 0;
+    rs.use_sel = K > 0;
+    rs.nwalk = K > 0 ? K + S : nt;
+    rs.nmc_max = std::min(nm, EXM_MAX_CHUNK);
+    rs.rc_cap = rs.rc = lags_by_taps(rs.nmc_max, rs.nwalk, ctx->ntau);
+    rs.nparts = exm_gather_parts_of(ctx->sm_count, (long long)ctx->nn * rs.nmc_max, rs.nmc_max, ctx->nn, rs.rc);
+    size_t by = 0;
+    for (const SlotNeed &n : slot_needs({nm, nt, nfreq, ctx->nn, ctx->ntau, ctx->sm_count, ctx->traj_fp64}, rs)) by += n.bytes;
+    by += (size_t)nm * nfreq * sizeof(float2) + (size_t)(ctx->nn + 1) * nm * sizeof(double) + (size_t)nm * 8 * 4;
+    return by + 2 * (size_t)rs.nmc_max * nt * sizeof(double2);
 }
 
 static RunShape run_shape(exm_ctx *ctx, int K, int S)
@@ -923,25 +1018,10 @@ static RunShape run_shape(exm_ctx *ctx, int K, int S)
     return rs;
 }
 
-static void ensure_slot(exm_ctx *ctx, exm_slot &sl, const RunShape &rs)
+static void ensure_slot(exm_ctx *ctx, exm_slot &sl, RunShape &rs)
 {
-    const size_t nmc = rs.nmc_max, nt = ctx->nt, nf = ctx->nfreq;
-    exm_ensure(ctx, sl.traj, 2 * nmc * nt * sizeof(float2));
-    if (ctx->traj_fp64) exm_ensure(ctx, sl.trajlo, 2 * nmc * nt * sizeof(float));
-    exm_ensure(ctx, sl.desc, 2 * nmc * nt * sizeof(double2));   // the filter's buffer before it holds descriptors
-    const size_t n_draws = rs.K > 0 ? (((size_t)ctx->nm * rs.S + EXM_MAX_REJ + 63) / 64) * 64 : 0;
-    exm_ensure(ctx, sl.keys, std::max<size_t>(rs.K > 0 ? nmc * nt : 1, n_draws) * sizeof(uint32_t));
-    exm_ensure(ctx, sl.picks, std::max<size_t>(1, (size_t)ctx->nm * rs.S) * sizeof(int32_t));
-    exm_ensure(ctx, sl.rej, (1 + EXM_MAX_REJ) * sizeof(int));
-    exm_ensure(ctx, sl.sel, std::max<size_t>(1, rs.use_sel ? nmc * rs.nwalk : 1) * sizeof(int32_t));
-    exm_ensure(ctx, sl.hist, (EXM_HB_N + 256) * sizeof(int));
-    exm_ensure(ctx, sl.win, (2 + EXM_MAX_NODES) * sizeof(int));
-    ensure_taps(ctx, sl, rs);
-    exm_ensure(ctx, sl.lamN, (size_t)(ctx->nn + 1) * ctx->nm * sizeof(double));
-    exm_ensure(ctx, sl.lnl, (size_t)ctx->nm * sizeof(double));
-    exm_ensure(ctx, sl.lnb, sizeof(double));
-    exm_ensure(ctx, sl.dev_err, sizeof(unsigned));
-    exm_ensure(ctx, sl.din, 6 * nf * sizeof(double) + 2 * nf * sizeof(float2) + 4 * sizeof(uint64_t));
+    ensure_needs(ctx, sl, rs, slot_needs);
+    const size_t nf = ctx->nfreq;
     const size_t hin = 6 * nf * sizeof(double) + 4 * sizeof(uint64_t);
     if (!sl.hostin.p || sl.hostin.bytes < hin) {
         if (sl.hostin.p) cudaFreeHost(sl.hostin.p);
@@ -1129,12 +1209,13 @@ extern "C" int exm_pe_intrinsic(exm_ctx *ctx, int n_seg, const double *d_H, cons
     REQUIRE(!ctx->shard, EXM_ERR_STATE, "a store shard gives node values (exm_node_values); ln Lambda needs every shard's");
     REQUIRE(n_seg >= 0 && d_H && d_L && sig2_H && sig2_L && ln_lambda && ln_b, EXM_ERR_ARG, "null argument");
     REQUIRE(n_loud == 0 || seeds, EXM_ERR_ARG, "seeds are needed when n_loud > 0");
-    const RunShape rs = run_shape(ctx, n_loud, n_random);
+    RunShape rs = run_shape(ctx, n_loud, n_random);
     exm_slot &sl = ctx->slot;
+    exm_fft_plan(ctx, 2 * rs.nmc_max);   // its work area first: what is left bounds the lags of a pass
     ensure_slot(ctx, sl, rs);
     std::vector<double> lnl(ctx->nm);
     const size_t nf = ctx->nfreq;
-    const bool graph = ctx->use_graph && ctx->nm <= rs.nmc_max && rs.rc >= ctx->ntau;
+    const bool graph = ctx->use_graph && ctx->nm <= rs.nmc_max && rs.rc_cap >= ctx->ntau;
     for (int e = 0; e < n_seg; ++e) {
         REQUIRE(rs.K == 0 || seeds[e] >= 0, EXM_ERR_ARG, "seed must be non-negative");
         const uint64_t seed = rs.K > 0 ? (uint64_t)seeds[e] : 0;
@@ -1162,7 +1243,7 @@ extern "C" int exm_pe_intrinsic(exm_ctx *ctx, int n_seg, const double *d_H, cons
 // later stage call).  They are always built anew: the filter and the trajectory upload share the descriptors' memory, and
 // the stage calls build descriptors of other shapes.  The caller's times are kept: walked if they are of this shape, else
 // put back after the build.
-static void tune_taps(exm_ctx *ctx, exm_slot &sl, const RunShape &rs, const ChunkInfo &ci)
+static void tune_taps(exm_ctx *ctx, exm_slot &sl, RunShape &rs, const ChunkInfo &ci)
 {
     const size_t nm = ctx->nm;
     const bool had_lo = sl.trajlo.p != nullptr;
@@ -1187,7 +1268,7 @@ static void tune_taps(exm_ctx *ctx, exm_slot &sl, const RunShape &rs, const Chun
         exm_run_topk(ctx, sl, ctx->nm, (const int *)ctx->d_order.p, rs.K, rs.S);
     }
     EXM_CUDA(cudaMemsetAsync(sl.dev_err.p, 0, sizeof(unsigned), ctx->stream));
-    exm_run_taps(ctx, sl, ci, 0, ctx->ntau, true);
+    exm_run_taps(ctx, sl, ci, 0, rs.rc, true);   // (the first pass, where the budget makes it several)
     if (draw && times) {
         EXM_CUDA(cudaMemcpyAsync(sl.sel.p, keep.data(), sizeof(int32_t) * keep.size(), cudaMemcpyHostToDevice,
                                  ctx->stream));
@@ -1203,8 +1284,8 @@ extern "C" int exm_autotune(exm_ctx *ctx, int n_loud, int n_random, int reps, in
     EXM_CUDA(cudaSetDevice(ctx->dev));
     REQUIRE(ctx->prep_ok, EXM_ERR_STATE, "exm_pe_prepare first");
     REQUIRE(ctx->ran_ok, EXM_ERR_STATE, "run exm_pe_intrinsic on this bank once first (the autotuner times the gather on its data)");
-    const RunShape rs = run_shape(ctx, n_loud, n_random);
-    REQUIRE(rs.nmc_max >= ctx->nm && rs.rc >= ctx->ntau, EXM_ERR_ARG,
+    RunShape rs = run_shape(ctx, n_loud, n_random);
+    REQUIRE(rs.nmc_max >= ctx->nm && rs.rc_cap >= ctx->ntau, EXM_ERR_ARG,
             "the autotuner needs the whole bank and every lag in one gather (bank <= 8192 templates)");
     exm_slot &sl = ctx->slot;
     ChunkInfo ci{0, ctx->nm, rs.nwalk, rs.use_sel, rs.lw};
@@ -1217,9 +1298,9 @@ extern "C" int exm_autotune(exm_ctx *ctx, int n_loud, int n_random, int reps, in
     const bool tim = ctx->tim_on;
     ctx->tim_on = false;
     auto time_gather = [&]() {
-        exm_run_gather_planes(ctx, sl, ci, 0, ctx->ntau);   // warm-up (and function attributes)
+        exm_run_gather_planes(ctx, sl, ci, 0, rs.rc);   // warm-up (and function attributes)
         EXM_CUDA(cudaEventRecord(e0, ctx->stream));
-        for (int r = 0; r < std::max(1, reps); ++r) exm_run_gather_planes(ctx, sl, ci, 0, ctx->ntau);
+        for (int r = 0; r < std::max(1, reps); ++r) exm_run_gather_planes(ctx, sl, ci, 0, rs.rc);
         EXM_CUDA(cudaEventRecord(e1, ctx->stream));
         EXM_CUDA(cudaEventSynchronize(e1));
         float ms = 0.f;
@@ -1290,6 +1371,7 @@ extern "C" int exm_filter(exm_ctx *ctx, const double *d_H, const double *d_L, co
     EXM_CUDA(cudaSetDevice(ctx->dev));
     RunShape rs = stage_shape(ctx, 0, 0);
     exm_slot &sl = ctx->slot;
+    exm_fft_plan(ctx, 2 * ctx->nm);
     ensure_slot(ctx, sl, rs);
     stage_input(ctx, sl, d_H, d_L, sig2_H, sig2_L);
     exm_run_filter(ctx, sl, (const float2 *)ctx->d_W.p, ctx->nm);
@@ -1498,7 +1580,6 @@ extern "C" int exm_node_values(exm_ctx *ctx, double *lamN_out)
         exm_run_taps(ctx, sl, ci, r0, rc, r0 == 0);
         exm_run_gather_planes(ctx, sl, ci, r0, rc);
     }
-    exm_ensure(ctx, sl.lamN, (size_t)(ctx->nn + 1) * ctx->nm * sizeof(double));
     exm_run_node_values(ctx, sl, 0, ctx->nm, (double *)sl.lamN.p);
     std::vector<double> h((size_t)(ctx->nn + 1) * ctx->nm);
     EXM_CUDA(cudaMemcpyAsync(h.data(), sl.lamN.p, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, ctx->stream));

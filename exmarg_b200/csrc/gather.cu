@@ -905,22 +905,33 @@ static int planes_tch_max(const exm_ctx *ctx, int wb)
 // the waits at each plane pair and the staging of its windows are paid once for all its templates), between
 // 256 and EXM_TCH_PLAN at 150, then the same for every chunk of a node.  2048 templates x 53 nodes at 352 / 512 / 704 /
 // 1024 / 2048: 75.5 / 70.9 / 68.0 / 65.4 ms, and on a later kernel 65.2 / 63.1 / 61.1 at the last three.
-static int planes_tch(const exm_ctx *ctx, const ChunkInfo &ci, int rc, int pct, int *maxn_out)
+static int planes_tch_of(int sm_count, long long pairs, int maxn, int rc, int pct)
 {
-    long long pairs = 0;
-    int maxn = 0;
-    for (int k = 0; k < ctx->nn; ++k) {
-        const int lo = std::max(ctx->mlo[k], ci.m_base), hi = std::min(ctx->mhi[k], ci.m_base + ci.nmc);
-        pairs += std::max(0, hi - lo);
-        maxn = std::max(maxn, hi - lo);
-    }
-    *maxn_out = maxn;
-    long long tch = pairs * rc / std::max(1, 8 * ctx->sm_count);
+    long long tch = pairs * rc / std::max(1, 8 * sm_count);
     tch = std::min<long long>(std::max<long long>(tch, 256), EXM_TCH_PLAN);
     tch = std::min<long long>(tch * pct / 150, EXM_TCH);
     tch = std::max<long long>(1, std::min<long long>(tch, maxn));
     const long long nch = std::max<long long>(1, (maxn + tch - 1) / tch);
     return (int)(((maxn + nch - 1) / nch + 15) / 16 * 16);
+}
+
+// (template, node) pairs of a pass over nmc templates from m_base, and the most of one node
+static long long planes_pairs(const exm_ctx *ctx, int m_base, int nmc, int *maxn_out)
+{
+    long long pairs = 0;
+    *maxn_out = 0;
+    for (int k = 0; k < ctx->nn; ++k) {
+        const int n = std::max(0, std::min(ctx->mhi[k], m_base + nmc) - std::max(ctx->mlo[k], m_base));
+        pairs += n;
+        *maxn_out = std::max(*maxn_out, n);
+    }
+    return pairs;
+}
+
+static int planes_tch(const exm_ctx *ctx, const ChunkInfo &ci, int rc, int pct, int *maxn_out)
+{
+    const long long pairs = planes_pairs(ctx, ci.m_base, ci.nmc, maxn_out);
+    return planes_tch_of(ctx->sm_count, pairs, *maxn_out, rc, pct);
 }
 
 // The windows' height and the descriptors' chunk, which the tap build and the gather share.  Rows: the most that
@@ -945,14 +956,19 @@ void exm_gather_plan(const exm_ctx *ctx, const ChunkInfo &ci, int rc, int *wb_ou
 // more when the launch has too few blocks to keep the SMs busy to the end.  Gather ms at 1 / 2 / 4 / 8 parts:
 // 3.5 waves of blocks (24 templates, every time) 1.22 / 1.05 / 0.97 / 1.00, (150 x 6 nodes) 1.66 / 1.49 / 1.45 / 1.50; 9.5
 // waves (333 x 21, two segments) 6.81 / 6.58 / 6.67 / 6.96; 15 waves (58 x 53) 1.92 / 1.93 / 2.04 / 2.28.
-int exm_gather_parts(const exm_ctx *ctx, int nmc, int m_base, int nwalk, int rc)
+int exm_gather_parts_of(int sm_count, long long pairs, int maxn, int nn, int rc)
+{
+    const int tch = std::max(16, planes_tch_of(sm_count, pairs, maxn, rc, 150));
+    const long long blocks = (long long)rc * nn * ((maxn + tch - 1) / std::max(tch, 1));
+    const long long waves = blocks / std::max(1, sm_count);
+    return waves >= 12 ? 1 : (waves >= 4 ? 2 : 4);
+}
+
+int exm_gather_parts(const exm_ctx *ctx, int nmc, int m_base, int rc)
 {
     int maxn = 0;
-    const ChunkInfo ci{m_base, nmc, nwalk, 0, 0.f};
-    const int tch = std::max(16, planes_tch(ctx, ci, rc, 150, &maxn));
-    const long long blocks = (long long)rc * ctx->nn * ((maxn + tch - 1) / std::max(tch, 1));
-    const long long waves = blocks / std::max(1, ctx->sm_count);
-    return waves >= 12 ? 1 : (waves >= 4 ? 2 : 4);
+    const long long pairs = planes_pairs(ctx, m_base, nmc, &maxn);
+    return exm_gather_parts_of(ctx->sm_count, pairs, maxn, ctx->nn, rc);
 }
 
 void exm_run_gather_planes(exm_ctx *ctx, exm_slot &sl, const ChunkInfo &ci, int r0, int rc)

@@ -220,11 +220,13 @@ struct ChunkInfo {
     int use_sel;  // sel holds the walked times
     float lw;     // log weight of a random draw
 };
-int exm_tap_parts(const exm_ctx *ctx, int nmc, int nwalk, int rc);
+int exm_tap_parts(int sm_count, int nmc, int nwalk, int rc);
 void exm_run_taps(exm_ctx *ctx, exm_slot &sl, const ChunkInfo &ci, int r0, int rc, bool first_chunk_of_lags);
 void exm_run_gather_planes(exm_ctx *ctx, exm_slot &sl, const ChunkInfo &ci, int r0, int rc);
 void exm_gather_plan(const exm_ctx *ctx, const ChunkInfo &ci, int rc, int *wb, int *ng);
-int exm_gather_parts(const exm_ctx *ctx, int nmc, int m_base, int nwalk, int rc);
+int exm_gather_parts(const exm_ctx *ctx, int nmc, int m_base, int rc);
+int exm_gather_parts_of(int sm_count, long long pairs, int maxn, int nn, int rc);
+size_t exm_workspace_bytes(const exm_ctx *ctx, int nm, int nt, int nfreq, int K, int S);
 void exm_make_tmap(exm_ctx *ctx, int wb);
 int exm_gather_num_cfgs();
 void exm_run_node_lse(exm_ctx *ctx, exm_slot &sl, int m_base, int nmc);

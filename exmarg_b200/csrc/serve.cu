@@ -94,21 +94,11 @@ struct exm_server {
     std::thread dispatcher;
 };
 
-// device bytes one worker's workspace takes for a bank (as exm_pe_intrinsic sizes it): the FFT rows and
-// trajectories, selection, tap descriptors, partial sums and the bank, plus cuFFT's work area
+// device bytes one worker takes for a bank, with a margin (until a worker of it has run and was measured)
 static size_t workspace_estimate(const exm_server *s, const SrvBank &b)
 {
-    const exm_ctx *p = s->parent;
-    const size_t nm = b.nm, nt = b.nt, nmc = std::min<size_t>(nm, EXM_MAX_CHUNK);
-    const size_t nwalk = s->n_loud > 0 ? (size_t)(s->n_loud + s->n_random) : nt;
-    const size_t per_lag = nmc * nwalk * 20;
-    const size_t rc = std::max<size_t>(1, std::min<size_t>((size_t)p->ntau, ((size_t)8 << 30) / std::max<size_t>(per_lag, 1)));
-    size_t by = 2 * nmc * nt * (16 + 8 + 4);   // FFT rows, trajectories, ln|z| residuals
-    by += std::max(nmc * nt, nm * 1024 + 4096) * 4 + nm * 1024 * 4;
-    by += nmc * nwalk * 4 + rc * 48 * (nmc + 1) * 4 + rc * per_lag;
-    by += (size_t)(p->nn + 1) * p->ntau * nm * 8 + nm * 8 * 12 + nm * (size_t)b.nfreq * 8;
-    by += 2 * nm * nt * 16 / std::max<size_t>(1, nm / std::max<size_t>(nmc, 1));
-    return (size_t)((double)by * 1.05) + ((size_t)64 << 20);
+    return (size_t)((double)exm_workspace_bytes(s->parent, b.nm, b.nt, b.nfreq, s->n_loud, s->n_random) * 1.05) +
+           ((size_t)64 << 20);
 }
 
 static void worker_main(exm_server *s, SrvWorker *w);

@@ -527,11 +527,11 @@ __global__ void __launch_bounds__(1024) k_windows(const int *hist_b, const int *
 
 // Parts of the walked times in the count: as many as give each SM about 16 warps of lags, of at least 64 times (more
 // parts cost more than they bring: every part writes its own counts, each to a sector of its own)
-int exm_tap_parts(const exm_ctx *ctx, int nmc, int nwalk, int rc)
+int exm_tap_parts(int sm_count, int nmc, int nwalk, int rc)
 {
     const long long warps = (long long)nmc * ((rc + 31) / 32);
     long long nq = 1;
-    while (nq < 32 && warps * nq < 16LL * ctx->sm_count && nwalk / (2 * nq) >= 64) nq *= 2;
+    while (nq < 32 && warps * nq < 16LL * sm_count && nwalk / (2 * nq) >= 64) nq *= 2;
     return (int)nq;
 }
 
@@ -562,7 +562,7 @@ void exm_run_taps(exm_ctx *ctx, exm_slot &sl, const ChunkInfo &ci, int r0, int r
     a.use_sel = ci.use_sel;
     a.r0 = r0;
     a.rc = rc;
-    a.nq = exm_tap_parts(ctx, ci.nmc, ci.nwalk, rc);
+    a.nq = exm_tap_parts(ctx->sm_count, ci.nmc, ci.nwalk, rc);
     a.cq = a.cnt + (size_t)rc * EXM_NPAIR * (ci.nmc + 1);
     a.hstep = (long long)ci.nmc * ci.nwalk > (1 << 18) ? 8 : 1;   // enough samples to place the windows
     a.want_hb = first_chunk_of_lags ? 1 : 0;

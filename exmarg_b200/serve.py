@@ -30,15 +30,25 @@ from .store import upload_store
 
 def workspace_bytes(nm, n_time, n_nodes, n_lags, nfreq, nwalk):
     """device bytes one worker's workspace takes for a bank of nm templates (as exm_pe_intrinsic
-    sizes it): FFT and trajectories, selection, tap descriptors, partial sums, bank copies"""
+    sizes it), with a margin: trajectories, selection, tap descriptors (the FFT rows before them in the same
+    memory), partial sums, bank copies, cuFFT's work area"""
+    sms = 148
     nmc = min(nm, 8192)
-    per_lag = nmc * nwalk * 20
-    rc = max(1, min(n_lags, (8 << 30) // max(per_lag, 1)))
-    b = 2 * nmc * n_time * (16 + 8 + 4)                  # FFT buffer + trajectories + ln|z| residuals
+    rc = max(1, min(n_lags, (8 << 30) // max(nmc * nwalk * 20, 1)))
+    # every (plane pair, template) run of descriptors is padded to groups of four, a lag's to chunks of 512
+    pitch = -(-(nmc * nwalk + 3 * nmc * min(48, nwalk)) // 512) * 512
+    parts = 1                                            # of the walked times in the count
+    while parts < 32 and nmc * -(-rc // 32) * parts < 16 * sms and nwalk // (2 * parts) >= 64:
+        parts *= 2
+    tch = min(max(n_nodes * nmc * rc // (8 * sms), 256), 2048, nmc)
+    waves = rc * n_nodes * -(-nmc // tch) // sms
+    sums = 1 if waves >= 12 else 2 if waves >= 4 else 4  # partial sums per (node, lag, template)
+    b = max(2 * nmc * n_time * 16, rc * pitch * 16) + rc * pitch * 4
+    b += 2 * nmc * n_time * (8 + 4)                      # trajectories + ln|z| residuals
     b += max(nmc * n_time, nm * 1024 + 4096) * 4 + nm * 1024 * 4
-    b += nmc * nwalk * 4 + rc * 48 * (nmc + 1) * 4 + rc * per_lag
-    b += (n_nodes + 1) * n_lags * nm * 8 + nm * 8 * 12 + nm * nfreq * 8
-    b += 2 * nm * n_time * 16 // max(1, nm // max(nmc, 1))  # cuFFT work area (about one buffer)
+    b += nmc * nwalk * 4 + rc * 48 * (nmc + 1 + (parts * nmc if parts > 1 else 0)) * 4
+    b += (n_nodes + 1) * nm * 8 * (n_lags * sums + 2) + nm * 8 * 12 + nm * nfreq * 8
+    b += 2 * nmc * n_time * 16                           # cuFFT work area (about one buffer)
     return int(b * 1.05) + (64 << 20)
 
 
