@@ -263,7 +263,7 @@ extern "C" int exm_w_build(exm_ctx *ctx, int n_nodes, const double *s_nodes, int
             }
         }
         const size_t nW = (size_t)n_nodes * n_tau * n_keys;
-        dbuf d_s, d_c2p, d_s2p, d_ap, d_cg, d_wq, d_resp, d_scale, d_W, d_out, d_tiles, d_l1, d_l2, d_dph, d_cm, d_bw, d_bad;
+        dbuf d_s, d_c2p, d_s2p, d_ap, d_cg, d_wq, d_resp, d_scale, d_W, d_out, d_tiles, d_l1, d_l2, d_dph, d_bw, d_bad;
         struct Guard {
             exm_ctx *c;
             std::vector<dbuf *> b;
@@ -273,7 +273,7 @@ extern "C" int exm_w_build(exm_ctx *ctx, int n_nodes, const double *s_nodes, int
                     if (x->p) exm_free(c, *x);
             }
         } guard{ctx, {&d_s, &d_c2p, &d_s2p, &d_ap, &d_cg, &d_wq, &d_resp, &d_scale, &d_W, &d_out, &d_tiles, &d_l1,
-                      &d_l2, &d_dph, &d_cm, &d_bw, &d_bad}};
+                      &d_l2, &d_dph, &d_bw, &d_bad}};
         auto up = [&](dbuf &b, const void *src, size_t bytes) {
             exm_alloc(ctx, b, bytes);
             exm_copy_in(ctx, b.p, src, bytes);
@@ -288,11 +288,11 @@ extern "C" int exm_w_build(exm_ctx *ctx, int n_nodes, const double *s_nodes, int
         up(d_scale, scale, (size_t)n_nodes * n_keys * sizeof(double));
         up(d_tiles, tiles.data(), tiles.size() * sizeof(int4));
         exm_alloc(ctx, d_W, nW * sizeof(double));
-        exm_alloc(ctx, d_out, nW * sizeof(float));
+        // the result's memory holds a pixel's cosines until the last product is done
+        exm_alloc(ctx, d_out, std::max(nW * sizeof(float), (size_t)(n_max + 1) * Qp * sizeof(double)));
         exm_alloc(ctx, d_l1, (size_t)nl * Qp * sizeof(double));
         exm_alloc(ctx, d_l2, (size_t)nl * Qp * sizeof(double));
         exm_alloc(ctx, d_dph, (size_t)Qp * sizeof(double));
-        exm_alloc(ctx, d_cm, (size_t)(n_max + 1) * Qp * sizeof(double));
         exm_alloc(ctx, d_bw, (size_t)n_nodes * Qp * sizeof(double));
         exm_alloc(ctx, d_bad, sizeof(unsigned long long));
         EXM_CUDA(cudaMemsetAsync(d_W.p, 0, nW * sizeof(double), ctx->stream));
@@ -307,7 +307,7 @@ extern "C" int exm_w_build(exm_ctx *ctx, int n_nodes, const double *s_nodes, int
             exm_allow_smem(ctx, (const void *)k_w_gemm<RG, R>, w_smem(RG, R));
             k_w_gemm<RG, R><<<(int)tiles.size(), kWThreads, w_smem(RG, R), ctx->stream>>>(
                 (const int4 *)d_tiles.p, Qp, n_nodes, n_max, (const double *)d_l1.p, (const double *)d_l2.p,
-                (const double *)d_cm.p, (const double *)d_bw.p, j0[p], w[2 * p], w[2 * p + 1], n_tau, n_keys,
+                (const double *)d_out.p, (const double *)d_bw.p, j0[p], w[2 * p], w[2 * p + 1], n_tau, n_keys,
                 (double *)d_W.p);
         };
         for (int p = 0; p < n_pix; ++p) {
@@ -318,7 +318,7 @@ extern "C" int exm_w_build(exm_ctx *ctx, int n_nodes, const double *s_nodes, int
                                                                 (const double *)d_s.p, nl, Qp, (double *)d_l1.p,
                                                                 (double *)d_l2.p, (double *)d_dph.p, (double *)d_bw.p);
             k_w_cos<<<dim3((Qp + 127) / 128, n_max + 1), 128, 0, ctx->stream>>>((const double *)d_dph.p, Qp,
-                                                                               (double *)d_cm.p);
+                                                                               (double *)d_out.p);
             // the fewest rows that hold the nodes: one row group up to 8 nodes, else 5 to 8 rows in each of 2, 4 or 8
             const int rg = n_nodes <= 8 ? 1 : n_nodes <= 16 ? 2 : n_nodes <= 32 ? 4 : 8;
             auto rows = [&](auto r) {
