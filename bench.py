@@ -158,9 +158,9 @@ def measured_peaks():
 # read per node-tap both do), so the full launch's traffic is this figure times its node-taps.  The capture
 # holds only for the kernel sources it was taken on: if they changed since, traffic is reported as null.
 GATHER_TRAFFIC = {
-    "dram_bytes_per_node_tap": 8.6897,       # (4.1217e9 + 8.65e6) B / 4.7531e8 node-taps (20 warps x 2)
-    "l2_read_hit_rate": 64.13,             # lts__t_sector_op_read_hit_rate.pct
-    "sources_sha256": "e3ad869d64ebbd1aaf4fec5c123e9433565c1b6a64cb17609788c3620331658d",
+    "dram_bytes_per_node_tap": 8.6874,       # (4.1213e9 + 7.89e6) B / 4.7531e8 node-taps (20 warps x 2)
+    "l2_read_hit_rate": 64.08,             # lts__t_sector_op_read_hit_rate.pct
+    "sources_sha256": "4868871de6990284f2f4fed29900ac52cc0c8cf0d7cfbc3122f8a02cfd238ced",
     "capture": "profiles/k_gather_planes_small.md",
 }
 GATHER_SOURCES = ("exmarg_b200/csrc/gather.cu", "exmarg_b200/csrc/taps.cu", "exmarg_b200/csrc/kernels.cuh")
@@ -982,6 +982,10 @@ def run_b200(args):
     peak, peak_kind = measured_peaks()
     achieved = bytes_per_launch / (g_ms / 1000.0) / 1e9
     node_taps_launch = tm["node_taps"] / max(launches, 1)
+    # the gather's first limit is the shared memory it reads its 8 table values a node-tap from: 128 bytes a clock and
+    # each of the 148 SMs where a warp's reads fall on different banks
+    smem_gbs = 32.0 * node_taps_launch / (g_ms / 1000.0) / 1e9
+    smem_peak = 128.0 * 148 * clk["sm_mhz"] / 1e3 if clk.get("sm_mhz") else None
     traffic, l2_hit, traffic_why = gather_traffic(node_taps_launch)
     dram_gbs = (traffic / (g_ms / 1000.0) / 1e9) if traffic else None
     line = {"metric": METRIC, "value": value, "unit": "segments/s", "n_gpus": world, "steps": args.steps,
@@ -996,9 +1000,12 @@ def run_b200(args):
             "boundary_taps_per_step": tm["boundary_taps"] / args.steps,
             "stages_ms_per_step": {k: tm[k] / args.steps for k in ("filter_ms", "select_ms", "taps_ms", "gather_ms",
                                                                     "epilogue_ms")},
-            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                         "achieved_is": "logical gather bytes (32 B per node-tap + 16 B of trajectory per tap) per "
-                                        "launch / CUDA-event launch time; served from shared memory, not DRAM",
+            "roofline": {"bound": "shared memory", "achieved": smem_gbs, "peak": smem_peak, "unit": "GB/s",
+                         "frac": smem_gbs / smem_peak if smem_peak else None,
+                         "achieved_is": "table values read from the staged windows (8 per node-tap) per launch / "
+                                        "CUDA-event launch time",
+                         "peak_is": "128 B a clock and SM without bank conflicts, at the sampled SM clock (nominal)",
+                         "hbm_peak": peak, "frac_logical_of_hbm": achieved / peak,
                          "traffic": traffic, "traffic_is": "ncu dram read + write bytes per node-tap of a reduced "
                                                            "case x this launch's node-taps" if traffic else traffic_why,
                          "achieved_dram": dram_gbs, "frac_dram": (dram_gbs / peak) if dram_gbs else None,
@@ -1084,7 +1091,7 @@ def main():
     ap.add_argument("--lags", type=int, default=87, help="table lags (reduced profiling cases; odd)")
     ap.add_argument("--gather-cfg", type=int, default=-1, help="force a gather launch shape (no autotuning)")
     ap.add_argument("--gather-chunk-pct", type=int, default=0,
-                    help="with --gather-cfg: templates per gather block in percent of the default (0: 100)")
+                    help="with --gather-cfg: templates per gather block (150: the library's own choice, others in proportion; 0: 150)")
     ap.add_argument("--prec-templates", type=int, default=64,
                     help="templates of the float64 oracle sample of the 16-bit table legs (0: no such legs)")
     ap.add_argument("--prec-steps", type=int, default=5, help="timed segments of each 16-bit table leg")

@@ -490,8 +490,8 @@ class Context:
         return best.value, ms
 
     def set_gather_cfg(self, cfg, chunk_pct=0):
-        """launch shape (index into GATHER_SHAPES) and templates per block in percent of the default
-        (0 keeps the current)"""
+        """launch shape (index into GATHER_SHAPES) and templates per block (150: the library's own
+        choice, others in proportion; 0 keeps the current)"""
         self._check(self.lib.exm_set_gather_cfg(self.h, int(cfg), int(chunk_pct)))
         self.gather_cfg = int(cfg)
         if chunk_pct:

@@ -1307,7 +1307,7 @@ extern "C" int exm_autotune(exm_ctx *ctx, int n_loud, int n_random, int reps, in
         EXM_CUDA(cudaEventElapsedTime(&ms, e0, e1));
         return ms / std::max(1, reps);
     };
-    // 1: every launch shape with the default template chunk
+    // 1: every launch shape, at two thirds of the library's own templates per block
     double best = 1e300;
     int arg = keep;
     ctx->gather_chunk_pct = 100;
@@ -1320,7 +1320,7 @@ extern "C" int exm_autotune(exm_ctx *ctx, int n_loud, int n_random, int reps, in
             arg = c;
         }
     }
-    // 2: the templates per gather block (percent of the one-wave-per-lag size) with the best shape
+    // 2: the templates per gather block (150: the library's own choice) with the best shape
     static const int pcts[] = {50, 150, 200};
     int best_pct = 100;
     ctx->gather_cfg = arg;

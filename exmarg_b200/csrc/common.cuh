@@ -152,14 +152,13 @@ struct exm_ctx {
     dbuf d_ckd;                       // double [EXM_MAX_NODES]: ck
     dbuf d_stats;                     // uint64 [4]: gather counters (slow-path taps, boundary taps)
 
-    // launch shape of the plane gather (index into its table; chosen by exm_autotune)
     exm_hostio *hostio = nullptr;        // made by the first large copy from or to pageable memory
     struct exm_redshift *rs = nullptr;   // pe_redshift's grid and buffers (csrc/redshift.cu)
-    int gather_cfg = 0;
-    int gather_chunk_pct = 150;
-    bool test_wait_expiry = false;
+    int gather_cfg = 0;              // launch shape of the plane gather (index into its table; chosen by exm_autotune)
+    int gather_chunk_pct = 150;      // templates per gather block: 150 the library's own choice, others in proportion
+    bool test_wait_expiry = false;   // the plane gather stages nothing and its barrier waits run out (a test)
     bool traj_fp64 = false;          // filter precision 'fp64': the ln|z| residual is kept and used by the taps
-    exm_server *srv = nullptr;       // request loop served from this context (exm_serve_start)   // the plane gather stages nothing and its barrier waits run out (a test)   // templates per gather block, percent of the one-wave-per-lag size
+    exm_server *srv = nullptr;       // request loop served from this context (exm_serve_start)
 
     // cuFFT
     cufftHandle plan = 0;

@@ -14,7 +14,7 @@
 // path that reads the table from global memory.
 //
 // What bounds it (2048 templates x 53 nodes x 87 lags x 2048 times, 1.65e10 taps): shared-memory reads (eight a
-// tap, 79 % of the data pipe) and instruction issue (63 %) together; DRAM is at a tenth of its rate.  92.7 -> 61.3 ms:
+// tap, 79 % of the data pipe) and instruction issue (63 %) together; DRAM is at 0.36 of its rate.  92.7 -> 61.5 ms:
 //  * four taps of one template per group: the bookkeeping of templates, the ranges and the running maximum are paid
 //    once for four taps (5.4 -> 2.8 warp instructions per tap); padding the runs to whole groups adds 3.8 % taps;
 //  * a row pitch of a multiple of the 32 banks, and taps ordered so that a step's lanes hit different banks
@@ -23,7 +23,8 @@
 //    takes up to 2048 templates: every plane pair costs a block a fixed ~1.7 us of waits (planes_tch);
 //  * a warp's first descriptors and end templates of the next pair loaded before it waits for that pair's planes.
 //  * descriptors loaded by whole chunks: no lane's loads are predicated or replaced by constants (65.3 -> 62.7).
-// 20 warps at 96 registers: 16 warps 64.2 ms (too few to cover the latencies), 24 and 28 spill (68.4, 80).
+// 20 warps at 96 registers; with two thirds of the templates a block 63.9 ms, 16 warps 65.3 (too few to cover the
+// latencies), 24 warps 66.8 and 28 warps 78.8 (they spill).
 //
 // k_gather_simple (the gather_cpu / gather_gpu contract, any table per slot): one
 // block per (row, lag), the reference's arithmetic in float64.
@@ -203,12 +204,6 @@ __device__ __forceinline__ void interp_window(const TE *s0, const TE *s1, int o,
     const float t10 = TabElem<TE>::cvt(s0[o + WD]), t11 = TabElem<TE>::cvt(s0[o + WD + 1]);
     const float u00 = TabElem<TE>::cvt(s1[o]), u01 = TabElem<TE>::cvt(s1[o + 1]);
     const float u10 = TabElem<TE>::cvt(s1[o + WD]), u11 = TabElem<TE>::cvt(s1[o + WD + 1]);
-#ifdef EXM_SCALAR
-    const float a0 = t01 - t00, c0 = t10 - t00, e0 = (t11 - t10) - a0;
-    const float eps0 = fmaf(fd, a0, fbf * fmaf(fd, e0, c0));
-    const float a1 = u01 - u00, c1 = u10 - u00, e1 = (u11 - u10) - a1;
-    const float eps1 = fmaf(fd, a1, fbf * fmaf(fd, e1, c1));
-#else
     const f2_t p00 = f2_pack(t00, u00);
     const f2_t a = f2_sub(f2_pack(t01, u01), p00), c = f2_sub(f2_pack(t10, u10), p00);
     const f2_t e = f2_sub(f2_sub(f2_pack(t11, u11), f2_pack(t10, u10)), a);
@@ -216,7 +211,6 @@ __device__ __forceinline__ void interp_window(const TE *s0, const TE *s1, int o,
     const f2_t eps = f2_fma(fd2, a, f2_mul(fb2, f2_fma(fd2, e, c)));
     float eps0, eps1;
     f2_unpack(eps, eps0, eps1);
-#endif
     B = t00;
     E = fmaf(w, (u00 - t00) + (eps1 - eps0), eps0);
     if (!std::is_same<TE, float>::value) {
@@ -903,12 +897,12 @@ static int planes_tch_max(const exm_ctx *ctx, int wb)
 
 // templates per gather block: pct / 150 of the most that still gives every SM eight blocks (a block's start,
 // the waits at each plane pair and the staging of its windows are paid once for all its templates), between
-// 256 and EXM_TCH_PLAN at 150, then the same for every chunk of a node.  2048 templates x 53 nodes at 352 / 512 / 704 /
+// 256 and EXM_TCH at 150, then the same for every chunk of a node.  2048 templates x 53 nodes at 352 / 512 / 704 /
 // 1024 / 2048: 75.5 / 70.9 / 68.0 / 65.4 ms, and on a later kernel 65.2 / 63.1 / 61.1 at the last three.
 static int planes_tch_of(int sm_count, long long pairs, int maxn, int rc, int pct)
 {
     long long tch = pairs * rc / std::max(1, 8 * sm_count);
-    tch = std::min<long long>(std::max<long long>(tch, 256), EXM_TCH_PLAN);
+    tch = std::min<long long>(std::max<long long>(tch, 256), EXM_TCH);
     tch = std::min<long long>(tch * pct / 150, EXM_TCH);
     tch = std::max<long long>(1, std::min<long long>(tch, maxn));
     const long long nch = std::max<long long>(1, (maxn + tch - 1) / tch);

@@ -48,8 +48,7 @@ template <> struct TabElem<__nv_bfloat16> {
 inline size_t exm_dtype_bytes(int dtype) { return dtype == EXM_DTYPE_F32 ? 4 : 2; }
 inline int exm_dtype_wd(int dtype) { return dtype == EXM_DTYPE_F32 ? EXM_WD : EXM_WD16; }
 inline int exm_dtype_calign(int dtype) { return dtype == EXM_DTYPE_F32 ? 4 : 8; }
-#define EXM_TCH 2048        // templates per gather block
-#define EXM_TCH_PLAN 2048   // ... by default
+#define EXM_TCH 2048        // most templates per gather block
 
 // Tap descriptors of one lag are sorted by (plane pair, template) and each (pair, template) run is padded to
 // whole groups of EXM_GT taps, so that every group has one template.  They are stored in chunks of 32 EXM_GT ng
