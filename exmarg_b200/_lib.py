@@ -479,7 +479,8 @@ class Context:
                                                 int(nsel), int(ns), P(mass_ids), P(lna), P(tab_ids), P(out)))
 
     def autotune(self, n_loud=1024, n_random=1024, reps=2):
-        """time every launch shape of the plane gather on the last segment; keep the fastest.
+        """time every launch shape of the plane gather on the trajectories the context holds (after
+        pe_intrinsic on this bank); keep the fastest.
         returns (best index, ms per launch of each shape)"""
         best, pct = ctypes.c_int(), ctypes.c_int()
         ms = np.zeros(16, np.float64)

@@ -353,7 +353,8 @@ EXM_API int exm_select_times(exm_ctx *ctx, int64_t seed, int n_loud, int n_rando
 EXM_API int exm_np_exp32(exm_ctx *ctx, const float *x, float *y, int64_t n);
 
 /* Upload a time selection (nm, nwalk) from the host in place of exm_select_times
- * (nwalk = 0: every arrival time). */
+ * (nwalk = 0: every arrival time).  lw: 0, or the drawn times' log weight, any value common to
+ * them. */
 EXM_API int exm_set_times(exm_ctx *ctx, int nwalk, const int32_t *sel, const float *lw);
 
 /* The gather contract of exmarg/search/gather.py:114-140 / :340-371
